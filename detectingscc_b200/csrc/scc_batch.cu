@@ -56,7 +56,7 @@ __device__ void batch_one(Ex &ex, const BatchParams &p, uint32_t gi, char *base,
     }
     Graph g{bg.V, bg.E, p.Fr + bg.off_r, p.Fc + bg.off_c, p.Br + bg.off_r, p.Bc + bg.off_c, p.vec};
     if (threadIdx.x == 0) {
-        carve_work(base, bg.V, bg.E, HONG, &s_w);
+        carve_work(base, bg.V, bg.E, &s_w);
         s_w.qcap = p.qcap;
         s_w.bu_k = p.bu_k;
         s_w.pull_lane = PULL_LANE;
@@ -64,12 +64,11 @@ __device__ void batch_one(Ex &ex, const BatchParams &p, uint32_t gi, char *base,
     __syncthreads();
     const Work &w = s_w;
     ex.ctl = w.ctl;
-    // fresh control block and pivot table for this graph
+    // fresh control block and pivot word for this graph
     {
         uint32_t *c = reinterpret_cast<uint32_t *>(w.ctl);
         for (unsigned i = ex.tid(); i < sizeof(Ctl) / 4; i += ex.nthr()) c[i] = 0u;
-        const uint32_t npk = HONG ? 4u * (bg.V + 1u) + 8u : 1u;
-        for (uint32_t i = ex.tid(); i < npk; i += ex.nthr()) w.pivkey[i] = 0ull;
+        if (ex.leader()) w.pivkey[0] = 0ull;
         ex.sync();
         if constexpr (!Ex::cluster) ex.reset_counters();   // this CTA's counter ring and error flag
         if (ex.leader()) {
@@ -79,9 +78,9 @@ __device__ void batch_one(Ex &ex, const BatchParams &p, uint32_t gi, char *base,
         ex.sync();
     }
     ex.gl = 0u;
-    Carry cy{0u, 0u, 0u};
+    Carry cy{};
     int rc = HONG ? hong_front(ex, g, w, p.t1, p.t2, p.lw, cy) : slota_front(ex, g, w, p.t1, p.lw, cy);
-    if (rc == RUN_DONE) rc = HONG ? hong_loop(ex, g, w, cy, 0u) : slota_peels(ex, g, w, cy, 0u);
+    if (rc == RUN_DONE) rc = peel_loop(ex, g, w, cy, 0u);
     ex.sync();   // the same error word in every CTA of the policy
     const int err = *(volatile int *)&w.ctl->error;
     if (!err) {
@@ -415,7 +414,7 @@ extern "C" int scc_batch_create(scc_context *ctx, const scc_csr_view *graphs, ui
     // largest graphs first (longest-processing-time order)
     rc = batch_upload_order(b, b->cluster, b->big_vertices);
     if (rc != SCC_OK) { batch_free(b); return rc; }
-    b->scratch_per_cta = carve_work(nullptr, b->maxV, b->maxE, true, nullptr);
+    b->scratch_per_cta = carve_work(nullptr, b->maxV, b->maxE, nullptr);
     rc = batch_reserve_scratch(b, b->threads, b->qcap, b->cluster, b->nbig);
     if (rc != SCC_OK) { batch_free(b); return rc; }
     *out = b;

@@ -27,7 +27,7 @@ constexpr uint32_t DEAD = 0x3FFFFFFFu;
 constexpr uint32_t FVB = 0x40000000u;
 constexpr uint32_t BVB = 0x80000000u;
 constexpr uint32_t FULL = 0xFFFFFFFFu;
-constexpr uint32_t MAX_V = 0x0FFFFFFEu;   // 4V+3 split names must stay below DEAD
+constexpr uint32_t MAX_V = 0x0FFFFFFEu;   // ids fit a state word's range bits and a colour word
 // label[v] with this bit set holds v's canonical label itself (the low
 // bits): a vertex that is its own SCC (trim-1, trim-2, small residual SCCs)
 // needs no smin entry and no gather when the labels are written out.
@@ -45,7 +45,7 @@ constexpr int E_NOT_CONVERGED = 21;
 constexpr int E_TIMEOUT = 22;
 constexpr int E_BAD_GRAPH = 23;
 
-enum { C_FQ = 0, C_BQ = 1, C_FH = 2, C_BH = 3, C_LIST = 4, C_FE = 5, C_BE = 6, C_RNG = 7, C_SCOPE = 8, NCNT = 9 };
+enum { C_FQ = 0, C_BQ = 1, C_FH = 2, C_BH = 3, C_LIST = 4, C_FE = 5, C_BE = 6, C_SCOPE = 7, NCNT = 8 };
 
 struct __align__(128) Ctl {
     // grid barrier arrival counter and the sticky error code share one
@@ -55,7 +55,7 @@ struct __align__(128) Ctl {
     int where; unsigned _p0[29];
     unsigned lc[3][NCNT];                          // per-pass counters, 3-slot ring
     unsigned maxdeg;                               // largest out- or in-degree (init sweep)
-    unsigned _p3[4];
+    unsigned _p3[7];
     unsigned long long n_trim1, n_trim2, n_pivot;
     unsigned long long t_edges, t_verts;           // instrumented work counters
     unsigned passes, outer;                        // passes run, peels / iterations
@@ -85,7 +85,7 @@ struct CtlReset {
 enum {
     PH_INIT = 1, PH_TRIM1_ONCE = 2, PH_TRIM1_APPLY = 3, PH_TRIM1_FIX = 4, PH_TRIM2 = 5, PH_TRIM2_APPLY = 6,
     PH_FIRST_PIVOT = 7, PH_BFS0 = 8, PH_BFS = 9, PH_PROP = 10, PH_HONG_UPDATE = 11, PH_SLOTA_FIRST_UPDATE = 12,
-    PH_SLOTA_PEEL_UPDATE = 13, PH_RENAME = 14, PH_PIVOTS = 15, PH_BFS_PULL = 16, PH_PROP_PULL = 17,
+    PH_PEEL_UPDATE = 13, PH_COMPACT = 14, PH_PEEL_SCC = 15, PH_BFS_PULL = 16, PH_PEEL_INIT = 17,
     PH_RES_TAG = 18, PH_RES_EXTRACT = 19, PH_RES_SOLVE = 20
 };
 
@@ -120,7 +120,8 @@ struct Work {
     uint32_t *Q[2][2];          // [direction][parity]
     uint2 *H[2][2];             // heavy chunks (vertex, chunk) [direction][parity]
     uint32_t hcap;
-    unsigned long long *pivkey; // Hong: 4V+4 slots; Slota: 1
+    uint2 *pc;                  // colour peels: (range, colour word) per vertex, over Q[1][0] and Q[1][1]
+    unsigned long long *pivkey; // the first pivot's key
     Ctl *ctl;
     uint32_t qcap;              // entries per CTA staging queue (dynamic shared memory)
     uint32_t bu_k;              // bottom-up BFS step when frontier edges > bu_k * scope vertices (0 = never)
@@ -134,13 +135,13 @@ constexpr uint32_t PULL_LANE = 32;   // Work::pull_lane of the batched and no-al
 // (nullptr: only count).  Returns the bytes used.  Same layout on host and
 // device; used by the batched form, where every CTA re-carves its private
 // scratch for each graph it takes.
-__host__ __device__ inline size_t carve_work(char *base, uint32_t V, uint32_t E, bool hong, Work *w)
+__host__ __device__ inline size_t carve_work(char *base, uint32_t V, uint32_t E, Work *w)
 {
     const size_t n1 = (size_t)V + 1;
     const size_t hcap = (size_t)E / CH + (size_t)E / HEAVY_T + 64;
     const size_t va = (n1 * 4 + 255) / 256 * 256;       // one vertex array
     const size_t ha = (hcap * 8 + 255) / 256 * 256;     // one chunk queue
-    const size_t pa = ((hong ? 4 * n1 + 8 : 1) * 8 + 255) / 256 * 256;
+    const size_t pa = 256;                              // the pivot word
     const size_t ca = (sizeof(Ctl) + 255) / 256 * 256;
     if (w && base) {
         w->st = (uint32_t *)(base);
@@ -154,6 +155,7 @@ __host__ __device__ inline size_t carve_work(char *base, uint32_t V, uint32_t E,
         w->Q[0][1] = (uint32_t *)(base + 7 * va);
         w->Q[1][0] = (uint32_t *)(base + 8 * va);
         w->Q[1][1] = (uint32_t *)(base + 9 * va);
+        w->pc = (uint2 *)w->Q[1][0];
         w->H[0][0] = (uint2 *)(base + 10 * va);
         w->H[0][1] = (uint2 *)(base + 10 * va + ha);
         w->H[1][0] = (uint2 *)(base + 10 * va + 2 * ha);
@@ -665,11 +667,10 @@ __device__ __forceinline__ bool stamp_claim(uint32_t *stamp, uint32_t u, uint32_
 // Load-balanced expansion of up to 32 adjacency lists held one per lane
 // (merge-path style): the warp walks the concatenation of the lists 32
 // entries at a time, each lane finds its owner by a 5-step binary search
-// over the exclusive scan of the degrees.  fn(valid, neighbour, aux_of_owner)
+// over the exclusive scan of the degrees.  fn(valid, neighbour, owner's lane)
 // is called by all lanes on every step.  Degrees must be <= HEAVY_T.
 template <class Fn>
-__device__ __forceinline__ unsigned lbs_expand(uint32_t beg, uint32_t deg, uint32_t aux,
-                                               const uint32_t *__restrict__ C, Fn &&fn)
+__device__ __forceinline__ unsigned lbs_walk(uint32_t beg, uint32_t deg, const uint32_t *__restrict__ C, Fn &&fn)
 {
     unsigned incl = warp_incl_scan(deg);
     unsigned total = __shfl_sync(FULL, incl, 31);
@@ -686,19 +687,17 @@ __device__ __forceinline__ unsigned lbs_expand(uint32_t beg, uint32_t deg, uint3
         }
         unsigned ex_o = __shfl_sync(FULL, excl, lo);
         unsigned beg_o = __shfl_sync(FULL, beg, lo);
-        unsigned aux_o = __shfl_sync(FULL, aux, lo);
         bool valid = e < total;
         uint32_t nbr = valid ? __ldg(&C[beg_o + (e - ex_o)]) : 0u;
-        fn(valid, nbr, aux_o);
+        fn(valid, nbr, lo);
     }
     return total;
 }
 
 // Same walk, two entries per lane per step so that each lane has two
-// independent gathers in flight: fn(v0, n0, aux0, v1, n1, aux1).
+// independent gathers in flight: fn(v0, n0, lane0, v1, n1, lane1).
 template <class Fn>
-__device__ __forceinline__ unsigned lbs_expand2(uint32_t beg, uint32_t deg, uint32_t aux,
-                                                const uint32_t *__restrict__ C, Fn &&fn)
+__device__ __forceinline__ unsigned lbs_walk2(uint32_t beg, uint32_t deg, const uint32_t *__restrict__ C, Fn &&fn)
 {
     unsigned incl = warp_incl_scan(deg);
     unsigned total = __shfl_sync(FULL, incl, 31);
@@ -717,13 +716,23 @@ __device__ __forceinline__ unsigned lbs_expand2(uint32_t beg, uint32_t deg, uint
         }
         const unsigned x0 = __shfl_sync(FULL, excl, lo0), x1 = __shfl_sync(FULL, excl, lo1);
         const unsigned b0 = __shfl_sync(FULL, beg, lo0), b1 = __shfl_sync(FULL, beg, lo1);
-        const unsigned a0 = __shfl_sync(FULL, aux, lo0), a1 = __shfl_sync(FULL, aux, lo1);
         const bool v0 = e0 < total, v1 = e1 < total;
         const uint32_t n0 = v0 ? __ldg(&C[b0 + (e0 - x0)]) : 0u;
         const uint32_t n1 = v1 ? __ldg(&C[b1 + (e1 - x1)]) : 0u;
-        fn(v0, n0, a0, v1, n1, a1);
+        fn(v0, n0, lo0, v1, n1, lo1);
     }
     return total;
+}
+
+// The same with one value per owner: fn(v0, n0, aux0, v1, n1, aux1).
+template <class Fn>
+__device__ __forceinline__ unsigned lbs_expand2(uint32_t beg, uint32_t deg, uint32_t aux,
+                                                const uint32_t *__restrict__ C, Fn &&fn)
+{
+    return lbs_walk2(beg, deg, C, [&](bool v0, uint32_t n0, unsigned l0, bool v1, uint32_t n1, unsigned l1) {
+        const uint32_t a0 = __shfl_sync(FULL, aux, l0), a1 = __shfl_sync(FULL, aux, l1);
+        fn(v0, n0, a0, v1, n1, a1);
+    });
 }
 
 // Fold member v into smin[rep] (the canonical label of rep's SCC): lanes
@@ -870,30 +879,11 @@ __device__ __forceinline__ unsigned long long pivot_key(const Graph &g, uint32_t
 }
 __device__ __forceinline__ uint32_t key_vertex(unsigned long long k) { return 0xFFFFFFFFu - (uint32_t)k; }
 
-// Range names after a FW-BW split: three fresh names per pivot.  The
-// reference uses 3*range + FV + 2*BV (scc_kernels.cu:138), which wraps.
-__device__ __forceinline__ uint32_t split_name(uint32_t V, uint32_t p, uint32_t s)
+// Ranges after the first FW-BW split: 1 neither, 2 forward only, 3 backward
+// only (the reference's 3*range + FV + 2*BV, scc_kernels.cu:138, for range 0).
+__device__ __forceinline__ uint32_t split_class(uint32_t s)
 {
-    return (V + 1u) + 3u * p + ((s & FVB) ? 1u : 0u) + ((s & BVB) ? 2u : 0u);
-}
-
-// Per-range atomicMax of pivot keys with warp aggregation over lanes that
-// share a range (match.any + redux) and a read before the atomic.
-// Returns true in exactly one lane of the whole launch per range: the one
-// whose atomicMax found the slot still empty (the range's first bid).
-__device__ __forceinline__ bool range_max_atomic(bool valid, uint32_t r, unsigned long long key,
-                                                 unsigned long long *pivkey)
-{
-    unsigned grp = __match_any_sync(FULL, valid ? r : 0xFFFFFFFFu);
-    unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-    unsigned mhi = __reduce_max_sync(grp, hi);
-    unsigned mlo = __reduce_max_sync(grp, hi == mhi ? lo : 0u);
-    bool first = false;
-    if (valid && lane_id() == (unsigned)(__ffs(grp) - 1)) {
-        unsigned long long k = ((unsigned long long)mhi << 32) | mlo;
-        if (k > *(volatile unsigned long long *)&pivkey[r]) first = atomicMax(&pivkey[r], k) == 0ull;
-    }
-    return first;
+    return 1u + ((s & FVB) ? 1u : 0u) + ((s & BVB) ? 2u : 0u);
 }
 
 }  // namespace sccb

@@ -99,9 +99,9 @@ __global__ void __launch_bounds__(GRID_THREADS, 1) k_scc_grid(Params p)
     if (blockIdx.x == 0 && threadIdx.x == 0) p.w.ctl->t_start = gtimer();
     bq_init();
     GridExec<INSTR> ex{p.w.ctl, 0u, p.pass_cap, p.hold};
-    Carry cy{0u, 0u, 0u};
+    Carry cy{};
     int rc = HONG ? hong_front(ex, p.g, p.w, p.t1, p.t2, p.lw, cy) : slota_front(ex, p.g, p.w, p.t1, p.lw, cy);
-    if (rc == RUN_DONE) rc = HONG ? hong_loop(ex, p.g, p.w, cy, p.tail_n) : slota_peels(ex, p.g, p.w, cy, p.tail_n);
+    if (rc == RUN_DONE) rc = peel_loop(ex, p.g, p.w, cy, p.tail_n);
     if (rc == RUN_RESIDUAL) {
         // the live vertices fit one CTA's shared memory: CTA 0 solves them
         // while the other CTAs write every other vertex's label (every SCC
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(GRID_THREADS, 1) k_scc_grid(Params p)
                                    p.g.V, (blockIdx.x - 1u) * blockDim.x + threadIdx.x, (gridDim.x - 1u) * blockDim.x);
             return;
         }
-        res_solve(p.g, p.w, p.w.L[cy.lsel], cy.nL, p.w.Q[1][(cy.gl - 1u) & 1u], last_count(ex, C_BQ), p.w.ctl,
+        res_solve(p.g, p.w, p.w.L[cy.lsel], cy.nL, p.w.Q[0][(cy.gl - 1u) & 1u], last_count(ex, C_BQ), p.w.ctl,
                   p.out);
         res_trace(p.w.ctl, cy.gl, cy.nL);
         if (threadIdx.x == 0) {
@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(GRID_THREADS, 1) k_scc_grid(Params p)
         if (threadIdx.x == 0) { p.w.ctl->tail_pass = cy.gl; p.w.ctl->nlive_tail = cy.nL; }
         BlockExec<INSTR> bx{p.w.ctl, cy.gl, p.pass_cap};
         bx.reset_counters();
-        if (HONG) hong_loop(bx, p.g, p.w, cy, 0u);
-        else slota_peels(bx, p.g, p.w, cy, 0u);
+        peel_loop(bx, p.g, p.w, cy, 0u);
         bx.gl = cy.gl;
         if (threadIdx.x == 0) p.w.ctl->passes = bx.gl;
         return;
@@ -153,9 +152,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) k_scc_block(Params p)
     bq_init();
     BlockExec<INSTR> ex{p.w.ctl, 0u, p.pass_cap};
     ex.reset_counters();
-    Carry cy{0u, 0u, 0u};
+    Carry cy{};
     int rc = HONG ? hong_front(ex, p.g, p.w, p.t1, p.t2, p.lw, cy) : slota_front(ex, p.g, p.w, p.t1, p.lw, cy);
-    if (rc == RUN_DONE) rc = HONG ? hong_loop(ex, p.g, p.w, cy, 0u) : slota_peels(ex, p.g, p.w, cy, 0u);
+    if (rc == RUN_DONE) rc = peel_loop(ex, p.g, p.w, cy, 0u);
     if (threadIdx.x == 0) p.w.ctl->passes = ex.gl;
     if (rc == RUN_DONE && p.out) {
         write_labels(p.w, p.g.V, p.out, threadIdx.x, blockDim.x);
@@ -255,7 +254,7 @@ WsLayout ws_layout(uint32_t V, uint32_t E)
     o.S0 = take(n1 * 4); o.S1 = take(n1 * 4);
     for (int i = 0; i < 4; i++) o.Q[i] = take(n1 * 4);
     for (int i = 0; i < 4; i++) o.H[i] = take(o.hcap * sizeof(uint2));
-    o.piv = take((4 * n1 + 8) * 8);
+    o.piv = take(8);
     o.ctl = take(sizeof(Ctl));
     o.need = need;
     return o;
@@ -294,6 +293,7 @@ int scc_ctx_reserve(scc_context *ctx, uint32_t V, uint32_t E)
     w.Q[0][1] = (uint32_t *)(b + o_Q[1]);
     w.Q[1][0] = (uint32_t *)(b + o_Q[2]);
     w.Q[1][1] = (uint32_t *)(b + o_Q[3]);
+    w.pc = (uint2 *)w.Q[1][0];   // Q[1][0] and Q[1][1] are adjacent
     w.H[0][0] = (uint2 *)(b + o_H[0]);
     w.H[0][1] = (uint2 *)(b + o_H[1]);
     w.H[1][0] = (uint2 *)(b + o_H[2]);
@@ -556,10 +556,10 @@ static int run_impl(scc_context *ctx, const scc_csr_view *gv, int algo, uint32_t
     const int ci = ctx->ctl_next;
     ctx->ctl_next = ci ^ 1;
     const CtlReset init{ctx->ctlb[ci ^ 1], (unsigned long long)ctx->timeout_ms * 1000000ull, ctx->dtrace,
-                        ctx->dtrace ? ctx->trace_cap : 0u, hong ? nullptr : ctx->work.pivkey};
+                        ctx->dtrace ? ctx->trace_cap : 0u, ctx->work.pivkey};
     const bool ready = ctx->ctl_ready[ci] && ctx->ctl_made[ci].timeout_ns == init.timeout_ns &&
                        ctx->ctl_made[ci].trace == init.trace && ctx->ctl_made[ci].trace_cap == init.trace_cap;
-    const bool piv_ready = ready && !hong && ctx->ctl_made[ci].pivkey == ctx->work.pivkey;
+    const bool piv_ready = ready && ctx->ctl_made[ci].pivkey == ctx->work.pivkey;
     ctx->ctl_ready[ci] = false;
     ctx->work.ctl = ctx->ctlb[ci];
     if (!ready) {
@@ -576,7 +576,7 @@ static int run_impl(scc_context *ctx, const scc_csr_view *gv, int algo, uint32_t
                                  ctx->work.ctl, st, dev ? nullptr : gv->Fc);
         if (rc != SCC_OK) return rc;
     }
-    if (!piv_ready) CK(cudaMemsetAsync(ctx->work.pivkey, 0, hong ? (4 * ((size_t)V + 1) + 8) * 8 : 8, st));
+    if (!piv_ready) CK(cudaMemsetAsync(ctx->work.pivkey, 0, 8, st));
 
 
     ctx->work.qcap = ctx->qcap;

@@ -24,7 +24,7 @@
 //   * every call shares the one array and overwrites it: calls whose work
 //     overlaps on the GPU (different streams, threads) race and must be
 //     serialised by the caller;
-//   * the control block and pivot table are cleared on every call
+//   * the control block and pivot word are cleared on every call
 //     (cudaMemsetAsync, which allocates nothing); no cudaMalloc, cudaFree,
 //     events or library allocator is used.
 #include <cuda_runtime.h>
@@ -49,10 +49,10 @@ constexpr size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 // Bytes the single-CTA kernel needs for a graph of V vertices and E edges
 // (the same arrays scc_run sizes per graph: vertex state, labels, stamps,
 // two live lists, four frontier queues, four heavy-chunk queues, the pivot
-// table and the control block).
+// word and the control block).
 constexpr size_t scratch_bytes(size_t V, size_t E)
 {
-    return al256((V + 1) * 4) * 10 + al256((E / CH + E / HEAVY_T + 64) * 8) * 4 + al256((4 * (V + 1) + 8) * 8) +
+    return al256((V + 1) * 4) * 10 + al256((E / CH + E / HEAVY_T + 64) * 8) * 4 + al256(8) +
            al256(sizeof(Ctl));
 }
 
@@ -189,12 +189,13 @@ extern "C" int scc_run_noalloc(const scc_csr_view *gv, int algo, uint32_t flags,
     w.Q[0][1] = (uint32_t *)take(n1 * 4);
     w.Q[1][0] = (uint32_t *)take(n1 * 4);
     w.Q[1][1] = (uint32_t *)take(n1 * 4);
+    w.pc = (uint2 *)w.Q[1][0];   // Q[1][0] and Q[1][1] are adjacent
     w.H[0][0] = (uint2 *)take(hcap * 8);
     w.H[0][1] = (uint2 *)take(hcap * 8);
     w.H[1][0] = (uint2 *)take(hcap * 8);
     w.H[1][1] = (uint2 *)take(hcap * 8);
     w.hcap = (uint32_t)hcap;
-    w.pivkey = (unsigned long long *)take((4 * n1 + 8) * 8);
+    w.pivkey = (unsigned long long *)take(8);
     w.ctl = (Ctl *)take(sizeof(Ctl));
     w.qcap = NOALLOC_QCAP;
     w.bu_k = 2;
@@ -205,7 +206,7 @@ extern "C" int scc_run_noalloc(const scc_csr_view *gv, int algo, uint32_t flags,
     Graph g{V, E, gv->Fr, gv->Fc ? gv->Fc : w.st, gv->Br, gv->Bc ? gv->Bc : w.st,
             ((((uintptr_t)gv->Fr) | ((uintptr_t)gv->Br)) & 15u) == 0u ? 1u : 0u};
     k_noalloc_ctl_init<<<1, 32, 0, st>>>(w.ctl, 4000ull * 1000000ull);
-    if (cudaMemsetAsync(w.pivkey, 0, hong ? (4 * n1 + 8) * 8 : 8, st) != cudaSuccess) {
+    if (cudaMemsetAsync(w.pivkey, 0, 8, st) != cudaSuccess) {
         cudaGetLastError();
         return SCC_ERR_CUDA;
     }

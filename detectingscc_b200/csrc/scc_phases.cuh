@@ -514,8 +514,8 @@ __device__ __forceinline__ void chunk_expand(Ex &ex, const uint32_t *__restrict_
 // queue 2): the scope of the next bottom-up step, which then walks only
 // those instead of the whole scope.
 template <class Ex>
-__device__ __forceinline__ void bfs_pull2(Ex &ex, const Graph &g, const Work &w, bool puf, bool pub, bool bw,
-                                          VList src, uint32_t k, unsigned par, unsigned nxt, uint32_t *sout)
+__device__ __forceinline__ void bfs_pull2(Ex &ex, const Graph &g, const Work &w, bool puf, bool pub, VList src,
+                                          uint32_t k, unsigned par, unsigned nxt, uint32_t *sout)
 {
     constexpr uint32_t MF = RMASK | FVB, MB = RMASK | BVB;
     uint32_t v[2], s[2], pos[4], end[4], want[4];
@@ -609,7 +609,7 @@ __device__ __forceinline__ void bfs_pull2(Ex &ex, const Graph &g, const Work &w,
         if (pub) bq_push(1u, found[2 * h + 1], v[h], w.qcap, w.Q[1][par], &ex.lc(nxt)[C_BQ], g.V, ex.ctl, 19);
         if (Ex::nbq > 2 && sout) {
             const bool fv = (s[h] & FVB) || found[2 * h], bv = (s[h] & BVB) || found[2 * h + 1];
-            const bool keep = s[h] != DEAD && !(fv && (bv || !bw));
+            const bool keep = s[h] != DEAD && !(fv && bv);
             bq_push(2u, keep, v[h], w.qcap, sout, &ex.lc(nxt)[C_SCOPE], g.V, ex.ctl, 25);
         }
     }
@@ -619,29 +619,11 @@ __device__ __forceinline__ void bfs_pull2(Ex &ex, const Graph &g, const Work &w,
     }
 }
 
-// Seed predicates for the first BFS pass.
-// A seed takes list entry x: operator() says whether it seeds, vert() which
-// vertex it seeds.
-struct SeedOne {      // the single first pivot
-    uint32_t p;
-    __device__ __forceinline__ bool operator()(const Work &, uint32_t v) const { return v == p; }
-    __device__ __forceinline__ uint32_t vert(const Work &, uint32_t x) const { return x; }
-};
-struct SeedRoot {     // colouring roots (selectPivotColoring, scc_kernels.cu:567-580)
-    __device__ __forceinline__ bool operator()(const Work &w, uint32_t v) const { return w.st[v] == v; }
-    __device__ __forceinline__ uint32_t vert(const Work &, uint32_t x) const { return x; }
-};
-struct SeedRanges {   // per-range pivots (selectPivots, scc_kernels.cu:4-19), walked over the
-                      // list of live ranges instead of every live vertex
-    __device__ __forceinline__ bool operator()(const Work &w, uint32_t r) const { return w.pivkey[r] != 0ull; }
-    __device__ __forceinline__ uint32_t vert(const Work &w, uint32_t r) const { return key_vertex(w.pivkey[r]); }
-};
-
-// Forward (and backward) reachability to closure.  Pass 0 walks src, tests
-// the seed predicate, flags seeds and expands them.  Each later pass picks,
-// per direction, top-down (expand the frontier queue and the heavy chunks)
-// or bottom-up over `scope` (the vertices the search can reach) when the
-// frontier's vertices have more than bu_k * scope.n edges to expand.  lw < 0 selects the
+// Forward and backward reachability from the first pivot p to closure.  Pass
+// 0 flags the pivot and expands it.  Each later pass picks, per direction,
+// top-down (expand the frontier queue and the heavy chunks) or bottom-up over
+// `scope` (the vertices the search can reach) when the frontier's vertices
+// have more than bu_k * scope.n edges to expand.  lw < 0 selects the
 // load-balanced warp schedule for top-down steps, lw >= 0 the virtual-warp
 // schedule with W = 1 << lw.
 //
@@ -651,67 +633,35 @@ struct SeedRanges {   // per-range pivots (selectPivots, scc_kernels.cu:4-19), w
 // rule weighs the frontier against it.  *last (optional) receives the scope
 // at the end: every live vertex of the original scope that is not visited
 // in both directions is in it.
-template <class Ex, class Seed>
-__device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, VList src, Seed seed, bool bw, int lw, VList scope,
-                       VList *last = nullptr)
+template <class Ex>
+__device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw, VList scope, VList *last = nullptr)
 {
     unsigned nshrink = 0;
     const unsigned gsz = (lw < 0) ? 32u : (32u >> lw);
-    const bool single = src.n == 1u && src.p == nullptr;
     bool ok = run_pass(ex, PH_BFS0, [&](unsigned, unsigned nxt) {
         const unsigned par = ex.gl & 1u;
-        const unsigned ng = single ? 0u : (src.n + gsz - 1u) / gsz;
-        const uint32_t bits = bw ? (FVB | BVB) : FVB;
-        if (single && seed(w, src.base)) {
-            // one seed (the first pivot, usually the largest hub): every warp
-            // takes CH-entry chunks of its out- and in-list in this pass
-            const uint32_t p = src.base;
-            if (ex.leader()) {
-                if (completed(atomicOr(&w.st[p], bits), bits, p) == p) atomicMin(cta_first_min(), p);
-                atomicAdd(&ex.ctl->n_pivot, 1ull);
-                w.smin[p] = p;   // p represents its SCC: the update passes fold the members in
-            }
-            // 64-entry pieces, one per warp, so the hub's lists spread over
-            // the whole grid in one round of gathers
-            const uint32_t r = w.st[p] & RMASK;
-            const uint32_t fb = __ldg(&g.Fr[p]), fe = __ldg(&g.Fr[p + 1]);
-            const uint32_t bb = bw ? __ldg(&g.Br[p]) : 0u, be = bw ? __ldg(&g.Br[p + 1]) : 0u;
-            const uint32_t nfc = (fe - fb + 63u) / 64u, nbc = (be - bb + 63u) / 64u;
-            for (uint32_t c = ex.wid(); c < nfc + nbc; c += ex.nwarps()) {
-                const int dir = c < nfc ? 0 : 1;
-                const uint32_t beg = dir ? bb + (c - nfc) * 64u : fb + c * 64u;
-                const uint32_t end = min(beg + 64u, dir ? be : fe);
-                const uint32_t *C = dir ? g.Bc : g.Fc;
-                const uint32_t e0 = beg + lane_id(), e1 = e0 + 32u;
-                const bool v0 = e0 < end, v1 = e1 < end;
-                const uint32_t n0 = v0 ? __ldg(&C[e0]) : 0u, n1 = v1 ? __ldg(&C[e1]) : 0u;
-                bfs_edge_visit2(ex, g, w, dir, v0, n0, r, v1, n1, r, par, nxt, true);
-                count_edges(ex, end - beg);
-            }
+        if (ex.leader()) {
+            if (completed(atomicOr(&w.st[p], FVB | BVB), FVB | BVB, p) == p) atomicMin(cta_first_min(), p);
+            atomicAdd(&ex.ctl->n_pivot, 1ull);
+            w.smin[p] = p;   // p represents its SCC: the update passes fold the members in
         }
-        for (uint32_t it = ex.wid(); it < ng; it += ex.nwarps()) {
-            unsigned slot = (lw < 0) ? lane_id() : (lane_id() >> lw);
-            uint32_t i = it * gsz + slot;
-            bool valid = i < src.n;
-            const uint32_t x = valid ? src.at(i) : 0u;
-            bool act = valid && seed(w, x);
-            uint32_t v = act ? seed.vert(w, x) : x;
-            bool lead = (lw <= 0) || ((lane_id() & ((1u << lw) - 1u)) == 0u);
-            uint32_t r = 0;
-            uint32_t done = 0xFFFFFFFFu;
-            if (act && lead) {
-                const uint32_t o = atomicOr(&w.st[v], bits);
-                done = completed(o, bits, v);
-                r = o & RMASK;
-                w.smin[v] = v;   // v represents its SCC from here on
-            }
-            fold_completed(done);
-            if (lw > 0) r = __shfl_sync(FULL, r, lane_id() & ~((1u << lw) - 1u));
-            unsigned m = __ballot_sync(FULL, act && lead);
-            if (lane_id() == 0 && m) atomicAdd(&ex.ctl->n_pivot, (unsigned long long)__popc(m));
-            count_verts(ex, valid && lead);
-            bfs_expand_lanes(ex, g, w, 0, v, act, r, lw, par, nxt);
-            if (bw) bfs_expand_lanes(ex, g, w, 1, v, act, r, lw, par, nxt);
+        // the pivot is usually the largest hub: 64-entry pieces of its out-
+        // and in-list, one per warp, so they spread over the whole grid in
+        // one round of gathers
+        const uint32_t r = w.st[p] & RMASK;
+        const uint32_t fb = __ldg(&g.Fr[p]), fe = __ldg(&g.Fr[p + 1]);
+        const uint32_t bb = __ldg(&g.Br[p]), be = __ldg(&g.Br[p + 1]);
+        const uint32_t nfc = (fe - fb + 63u) / 64u, nbc = (be - bb + 63u) / 64u;
+        for (uint32_t c = ex.wid(); c < nfc + nbc; c += ex.nwarps()) {
+            const int dir = c < nfc ? 0 : 1;
+            const uint32_t beg = dir ? bb + (c - nfc) * 64u : fb + c * 64u;
+            const uint32_t end = min(beg + 64u, dir ? be : fe);
+            const uint32_t *C = dir ? g.Bc : g.Fc;
+            const uint32_t e0 = beg + lane_id(), e1 = e0 + 32u;
+            const bool v0 = e0 < end, v1 = e1 < end;
+            const uint32_t n0 = v0 ? __ldg(&C[e0]) : 0u, n1 = v1 ? __ldg(&C[e1]) : 0u;
+            bfs_edge_visit2(ex, g, w, dir, v0, n0, r, v1, n1, r, par, nxt, true);
+            count_edges(ex, end - beg);
         }
         bq_flush(2, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], w.Q[1][par], &ex.lc(nxt)[C_BQ], g.V, ex.ctl,
                  &ex.lc(nxt)[C_FE], &ex.lc(nxt)[C_BE]);
@@ -739,7 +689,7 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, VList src, Seed se
         // expand than the scope has vertices to test (times bu_k)
         const uint32_t mf = last_count(ex, C_FE), mb = last_count(ex, C_BE);
         const bool puf = w.bu_k && (unsigned long long)mf > (unsigned long long)scope.n * w.bu_k;
-        const bool pub = bw && w.bu_k && (unsigned long long)mb > (unsigned long long)scope.n * w.bu_k;
+        const bool pub = w.bu_k && (unsigned long long)mb > (unsigned long long)scope.n * w.bu_k;
         unsigned cm = 3u;   // bit d: this pass tallies direction d
         if constexpr (skip_tally) {
             cm = 0u;
@@ -770,10 +720,10 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, VList src, Seed se
             const uint32_t isz = (lw < 0) ? gsz : (uint32_t)VWK * gsz;
             const uint32_t ngf = (nf + isz - 1u) / isz, ngb = (nb + isz - 1u) / isz;
             const uint32_t items_f = puf ? 0u : nhf + ngf;
-            const uint32_t items_b = pub ? 0u : (bw ? nhb + ngb : 0u);
+            const uint32_t items_b = pub ? 0u : nhb + ngb;
             for (uint32_t it = ex.wid(); it < nd + items_f + items_b; it += ex.nwarps()) {
                 if (it < nd) {
-                    bfs_pull2(ex, g, w, puf, pub, bw, psrc, it, par, nxt, sout);
+                    bfs_pull2(ex, g, w, puf, pub, psrc, it, par, nxt, sout);
                     continue;
                 }
                 const uint32_t it2 = it - nd;
@@ -830,100 +780,17 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, VList src, Seed se
 }
 
 // ---------------------------------------------------------------------
-// Label propagation over in-edges to a fixpoint:
-//   MAXP = true : colour = max id reachable (colorPropagation,
-//                 scc_kernels.cu:539-564, pulls the max over out-neighbours)
-//   MAXP = false: name = min id reachable (the "WCC" of propagateRange1 /
-//                 propagateRange2, scc_kernels.cu:496-536)
-// Written as a push over the reverse CSR: when w's value moves, its
-// in-neighbours are updated with atomicMax / atomicMin and queued.
-// ---------------------------------------------------------------------
-template <bool MAXP, class Ex>
-__device__ __forceinline__ void prop_visit(Ex &ex, const Graph &g, const Work &w, bool valid, uint32_t u,
-                                           uint32_t c, unsigned par, unsigned nxt, uint32_t tag)
-{
-    bool push = false;
-    if (valid) {
-        u = guard_id(u, g.V, ex.ctl);
-        uint32_t s = w.st[u];
-        if (MAXP) {
-            if (s < c) push = atomicMax(&w.st[u], c) < c && stamp_claim(w.stamp, u, tag);
-        } else {
-            if (s != DEAD && s > c) push = atomicMin(&w.st[u], c) > c && stamp_claim(w.stamp, u, tag);
-        }
-    }
-    bq_push(0, push, u, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 14);
-}
-
-template <bool MAXP, class Ex>
-__device__ bool ph_propagate(Ex &ex, const Graph &g, const Work &w, VList src0)
-{
-    uint32_t nq = 0, nh = 0;
-    bool first = true;
-    for (unsigned lev = 0;; lev++) {
-        if (lev > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 50); return false; }
-        bool ok = run_pass(ex, PH_PROP, [&](unsigned, unsigned nxt) {
-            const unsigned par = ex.gl & 1u, cp = par ^ 1u;
-            const uint32_t tag = ex.gl + 1u;
-            VList src = first ? src0 : VList{w.Q[0][cp], nq, 0u};
-            const uint32_t hn = first ? 0u : nh;
-            const uint32_t ng = (src.n + 31u) / 32u;
-            auto fn = [&](bool valid, uint32_t u, uint32_t c) { prop_visit<MAXP>(ex, g, w, valid, u, c, par, nxt, tag); };
-            auto fn2 = [&](bool v0, uint32_t u0, uint32_t c0, bool v1, uint32_t u1, uint32_t c1) {
-                prop_visit<MAXP>(ex, g, w, v0, u0, c0, par, nxt, tag);
-                prop_visit<MAXP>(ex, g, w, v1, u1, c1, par, nxt, tag);
-            };
-            for (uint32_t it = ex.wid(); it < hn + ng; it += ex.nwarps()) {
-                if (it < hn) {
-                    uint2 hc = w.H[0][cp][it];
-                    chunk_expand(ex, g.Br, g.Bc, hc, w.st[hc.x] & RMASK, fn2);
-                } else {
-                    uint32_t i = (it - hn) * 32u + lane_id();
-                    bool valid = i < src.n;
-                    uint32_t v = valid ? src.at(i) : 0u;
-                    uint32_t c = valid ? (w.st[v] & RMASK) : 0u;
-                    if (!MAXP && valid && c != v) {
-                        // pointer jumping: the name of v's name is also reachable from v
-                        // (the same fixpoint, reached in fewer sweeps on long chains)
-                        const uint32_t s2 = w.st[c];
-                        if (s2 != DEAD && (s2 & RMASK) < c) {
-                            c = s2 & RMASK;
-                            atomicMin(&w.st[v], c);
-                        }
-                    }
-                    uint32_t beg = 0, deg = 0;
-                    if (valid) { beg = __ldg(&g.Br[v]); deg = __ldg(&g.Br[v + 1]) - beg; }
-                    bool heavy = deg > HEAVY_T;
-                    warp_push_chunks(v, heavy ? (deg + CH - 1u) / CH : 0u, w.H[0][par],
-                                     &ex.lc(nxt)[C_FH], w.hcap, ex.ctl);
-                    if (heavy) deg = 0u;
-                    count_verts(ex, valid);
-                    count_edges(ex, lbs_expand(beg, deg, c, g.Bc, fn));
-                }
-            }
-            bq_flush(1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], nullptr, nullptr, g.V, ex.ctl);
-        });
-        if (!ok) return false;
-        first = false;
-        nq = last_count(ex, C_FQ);
-        nh = last_count(ex, C_FH);
-        if (nq + nh == 0u) return true;
-    }
-}
-
-// ---------------------------------------------------------------------
-// Hong update (scc_kernels.cu:124-142): FV and BV -> the SCC of the range's
-// pivot; otherwise the vertex moves to one of three fresh sub-range names
-// and is appended to the next live list.  With fold, the survivors also
-// bid for the pivot of their new range, which replaces the reference's
-// separate pollForPivots/selectPivots launches (scc_WCC.cu:860-862).
+// Hong's first update (scc_kernels.cu:124-142): FV and BV -> the SCC of the
+// first pivot p; otherwise the vertex moves to one of three sub-ranges
+// (forward only, backward only, neither: no SCC crosses them) and is
+// appended to the next live list.
 // ---------------------------------------------------------------------
 template <class Ex>
-__device__ bool ph_hong_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout,
-                               bool single, bool fold)
+__device__ bool ph_hong_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
 {
     return run_pass(ex, PH_HONG_UPDATE, [&](unsigned, unsigned nxt) {
-        uint32_t mn = 0xFFFFFFFFu;   // single: smallest member of the pivot's SCC seen by this thread
+        const uint32_t p = key_vertex(w.pivkey[0]);
+        uint32_t mn = 0xFFFFFFFFu;   // smallest member of the pivot's SCC seen by this thread
         for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
             uint32_t v[4], s[4];
             bool ok[4];
@@ -932,40 +799,29 @@ __device__ bool ph_hong_update(Ex &ex, const Graph &g, const Work &w, VList src,
             for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                bool surv = false, scc = false;
-                uint32_t p = 0u, nr = 0u;
+                bool surv = false;
                 if (s[j] != DEAD) {
-                    p = key_vertex(w.pivkey[single ? 0u : (s[j] & RMASK)]);
                     if ((s[j] & FVB) && (s[j] & BVB)) {
                         w.st[v[j]] = DEAD;
                         w.label[v[j]] = p;
-                        scc = true;
+                        mn = min(mn, v[j]);
                     } else {
-                        nr = split_name(g.V, p, s[j]);
-                        w.st[v[j]] = nr;
+                        w.st[v[j]] = split_class(s[j]);
                         surv = true;
                     }
                 }
-                if (single) mn = scc ? min(mn, v[j]) : mn;
-                else smin_fold(scc, p, v[j], w.smin);
-                bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
                 bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 15);
-                if (fold) {
-                    // the new ranges are listed by their first bid (as in ph_pivots)
-                    const bool first = range_max_atomic(surv, nr, surv ? pivot_key(g, v[j]) : 0ull, w.pivkey);
-                    warp_push(first, nr, w.Q[0][ex.gl & 1u], &ex.lc(nxt)[C_RNG], g.V + 1u, ex.ctl, 22);
-                }
             }
             count_verts_n(ex, (unsigned)ok[0] + ok[1] + ok[2] + ok[3]);
         }
-        if (single) block_min_atomic(mn, w.pivkey[0] ? &w.smin[key_vertex(w.pivkey[0])] : w.smin);
-        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl, &ex.lc(nxt)[C_FE]);
+        block_min_atomic(mn, w.pivkey[0] ? &w.smin[p] : w.smin);   // mn stays 0xFFFFFFFF without a pivot
+        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl);
     });
 }
 
-// Slota: the first FW-BW's SCC is final; every other live vertex starts
-// the colouring with colour = its own id (assignUniqueRange,
-// scc_kernels.cu:477-484) and is appended to the live list.
+// Slota: the first FW-BW's SCC is final; every other live vertex keeps
+// which of the two searches reached it as its range (no SCC crosses those)
+// and is appended to the live list of the colour peels.
 template <class Ex>
 __device__ bool ph_slota_first_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
 {
@@ -983,7 +839,7 @@ __device__ bool ph_slota_first_update(Ex &ex, const Graph &g, const Work &w, VLi
                 bool surv = false, scc = false;
                 if (s[j] != DEAD) {
                     if ((s[j] & FVB) && (s[j] & BVB)) { w.st[v[j]] = DEAD; w.label[v[j]] = p; scc = true; }
-                    else { w.st[v[j]] = v[j]; w.stamp[v[j]] = 0u; surv = true; }   // the colouring's work lists stamp them
+                    else { w.st[v[j]] = split_class(s[j]); surv = true; }
                 }
                 mn = scc ? min(mn, v[j]) : mn;
                 bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
@@ -1015,7 +871,7 @@ __device__ bool ph_slota_first_update_lazy(Ex &ex, const Graph &g, const Work &w
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const bool surv = s[j] != DEAD && (s[j] & (FVB | BVB)) != (FVB | BVB);
-                if (surv) { w.st[v[j]] = v[j]; w.stamp[v[j]] = 0u; }
+                if (surv) w.st[v[j]] = split_class(s[j]);
                 bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
                 bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 16);
             }
@@ -1027,27 +883,227 @@ __device__ bool ph_slota_first_update_lazy(Ex &ex, const Graph &g, const Work &w
     });
 }
 
-// Slota peel end (updateColoring, scc_kernels.cu:614-623; fwdColoring's
-// rangeSet, :607): visited vertices belong to their root's SCC; the rest
-// restart from their own colour and form the next live list.
+// Hong: the vertices left after the trims, compacted, with their out-arcs
+// tallied (the residual check).
 template <class Ex>
-__device__ bool ph_slota_peel_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
+__device__ bool ph_compact(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
 {
-    return run_pass(ex, PH_SLOTA_PEEL_UPDATE, [&](unsigned, unsigned nxt) {
+    return run_pass(ex, PH_COMPACT, [&](unsigned, unsigned nxt) {
         for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
             uint32_t v[4], s[4];
             bool ok[4];
             load_list4(src, base + 4u * lane_id(), v, ok);
 #pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : 0u;
+            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                bool surv = false, scc = false;
-                uint32_t c = 0u;
-                if (ok[j]) {
-                    if (s[j] & FVB) { c = s[j] & RMASK; w.st[v[j]] = DEAD; w.label[v[j]] = c; scc = true; }
-                    else { w.st[v[j]] = v[j]; surv = true; }
+                const bool surv = s[j] != DEAD;
+                bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
+                bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 18);
+            }
+            count_verts_n(ex, (unsigned)ok[0] + ok[1] + ok[2] + ok[3]);
+        }
+        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl, &ex.lc(nxt)[C_FE]);
+    });
+}
+
+// ---------------------------------------------------------------------
+// Colour peels: the SCCs of the vertices that the first FW-BW and the trims
+// leave, for all four drivers (the colouring loop of scc_Coloring.cu:590-637
+// and, with the same SCCs and counts, Hong's main loop scc_WCC.cu:851-930).
+// A peel gives every live vertex the largest id that reaches it (its colour),
+// finds the SCC of every colour's root -- the members of the colour that
+// reach the root -- and leaves the colours behind as ranges: no SCC crosses
+// two colours, so later peels walk no arc between them.  Peels alternate
+// between the forward and the reverse CSR ("reaches" and "is reached by"),
+// so both ends of a chain are cut.  The reference's loops drop the colours
+// after each peel (scc_Coloring.cu:614-623) and keep the direction, or split
+// each range by one pivot at a time (scc_WCC.cu:860-905): on a chain of
+// 6,278 SCCs (65,000 vertices, 418,172 arcs) that is 570 colour sweeps, or
+// 118 rounds with 1,450 BFS levels; kept colours need 8 peels, about 170
+// sweeps and levels together, and a third of the colour loop's arcs.  What
+// bounds them is the chain of dependent accesses of each level (list entry,
+// offsets and colour, arcs, neighbour's pair, atomic).  That graph, before
+// and now: one CTA vHong 26.5 -> 8.1 ms, vSlota 50.1 -> 6.8 ms; whole GPU
+// 18.6 -> 1.36 ms and 11.7 -> 1.26 ms.
+//
+// A live vertex's word pair pc[v]: x the range, y = (colour << 1) | flag.
+// One 8-byte gather per arc decides; a word of a vertex without colour is
+// all ones.  While colours spread, the flag says that v is in a work list
+// and not yet expanded (a raise finds it set and does not list v again;
+// taking v off the list clears it and reads the newest colour); it is clear
+// everywhere when they have settled, and then says that v reaches its root.
+// ---------------------------------------------------------------------
+
+// Vertices a warp takes at once from a list of n: the smallest power of two
+// that still gives every warp at most one item, at most 32.  A level's time
+// is the chain of dependent accesses of its longest item, so a short list is
+// spread over all warps before lanes are filled.
+template <class Ex>
+__device__ __forceinline__ uint32_t item_group(const Ex &ex, uint32_t n)
+{
+    uint32_t s = 32u;
+    while (s > 1u && (n + (s >> 1) - 1u) / (s >> 1) <= ex.nwarps()) s >>= 1;
+    return s;
+}
+
+// Word pairs of all vertices from their states (every state word is a range
+// class or final here).
+template <class Ex>
+__device__ bool ph_peel_init(Ex &ex, const Graph &g, const Work &w)
+{
+    return run_pass(ex, PH_PEEL_INIT, [&](unsigned, unsigned) {
+        for (uint32_t i0 = ex.tid() * 2u; i0 <= g.V; i0 += ex.nthr() * 2u) {
+            const bool two = i0 + 1u <= g.V;
+            uint2 s = make_uint2(DEAD, DEAD);
+            if (two) s = *reinterpret_cast<const uint2 *>(w.st + i0);
+            else s.x = w.st[i0];
+            const bool la = (s.x & (FVB | BVB)) == 0u && s.x != DEAD, lb = (s.y & (FVB | BVB)) == 0u && s.y != DEAD;
+            const uint4 o = make_uint4(la ? s.x : FULL, la ? (i0 << 1) | 1u : FULL, lb ? s.y : FULL,
+                                       lb ? ((i0 + 1u) << 1) | 1u : FULL);
+            if (two) *reinterpret_cast<uint4 *>(w.pc + i0) = o;
+            else w.pc[i0] = make_uint2(o.x, o.y);
+        }
+    });
+}
+
+// Two arcs per lane: the owner's colour c offered to neighbour n in range r.
+template <class Ex>
+__device__ __forceinline__ void peel_raise2(Ex &ex, const Graph &g, const Work &w, bool v0, uint32_t n0, uint32_t r0,
+                                            uint32_t c0, bool v1, uint32_t n1, uint32_t r1, uint32_t c1, unsigned par,
+                                            unsigned nxt)
+{
+    if (v0) n0 = guard_id(n0, g.V, ex.ctl);
+    if (v1) n1 = guard_id(n1, g.V, ex.ctl);
+    const uint2 a = v0 ? w.pc[n0] : make_uint2(FULL, FULL);
+    const uint2 b = v1 ? w.pc[n1] : make_uint2(FULL, FULL);
+    const bool t0 = v0 && a.x == r0 && (a.y >> 1) < c0;
+    const bool t1 = v1 && b.x == r1 && (b.y >> 1) < c1;
+    const uint32_t w0 = (c0 << 1) | 1u, w1 = (c1 << 1) | 1u;
+    const uint32_t o0 = t0 ? atomicMax(&w.pc[n0].y, w0) : FULL;
+    const uint32_t o1 = t1 ? atomicMax(&w.pc[n1].y, w1) : FULL;
+    // whoever sets the flag lists the vertex
+    bq_push(0, !(o0 & 1u) && o0 < w0, n0, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 14);
+    bq_push(0, !(o1 & 1u) && o1 < w1, n1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 14);
+}
+
+// Two arcs per lane: neighbour n joins the SCC of colour c's root.
+template <class Ex>
+__device__ __forceinline__ void peel_join2(Ex &ex, const Graph &g, const Work &w, bool v0, uint32_t n0, uint32_t c0,
+                                           bool v1, uint32_t n1, uint32_t c1, unsigned par, unsigned nxt)
+{
+    if (v0) n0 = guard_id(n0, g.V, ex.ctl);
+    if (v1) n1 = guard_id(n1, g.V, ex.ctl);
+    const bool t0 = v0 && w.pc[n0].y == c0 << 1;
+    const bool t1 = v1 && w.pc[n1].y == c1 << 1;
+    const uint32_t o0 = t0 ? atomicOr(&w.pc[n0].y, 1u) : 1u;
+    const uint32_t o1 = t1 ? atomicOr(&w.pc[n1].y, 1u) : 1u;
+    bq_push(0, !(o0 & 1u), n0, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 13);
+    bq_push(0, !(o1 & 1u), n1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 13);
+}
+
+// One fixpoint of a peel over (R, C): with RAISE the colours of the live
+// list spread, else the roots' SCCs are searched.  Lists longer than HEAVY_T
+// go through chunks, as in the first search.
+template <bool RAISE, class Ex>
+__device__ bool ph_peel_spread(Ex &ex, const Graph &g, const Work &w, VList L, const uint32_t *__restrict__ R,
+                               const uint32_t *__restrict__ C)
+{
+    uint32_t nq = L.n, nh = 0;
+    for (unsigned lev = 0;; lev++) {
+        if (lev > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, RAISE ? 50 : 40); return false; }
+        const bool ok = run_pass(ex, RAISE ? PH_PROP : PH_PEEL_SCC, [&](unsigned, unsigned nxt) {
+            const unsigned par = ex.gl & 1u, cp = par ^ 1u;
+            const uint32_t *src = lev == 0u ? L.p : w.Q[0][cp];
+            const uint32_t gs = item_group(ex, nq);
+            const uint32_t ng = (nq + gs - 1u) / gs;
+            for (uint32_t it = ex.wid(); it < nh + ng; it += ex.nwarps()) {
+                if (it < nh) {
+                    const uint2 hc = w.H[0][cp][it];
+                    const uint2 x = make_uint2(vld(&w.pc[hc.x].x), vld(&w.pc[hc.x].y));
+                    const uint32_t c = x.y >> 1;
+                    auto fn = [&](bool v0, uint32_t n0, uint32_t, bool v1, uint32_t n1, uint32_t) {
+                        if (RAISE) peel_raise2(ex, g, w, v0, n0, x.x, c, v1, n1, x.x, c, par, nxt);
+                        else peel_join2(ex, g, w, v0, n0, c, v1, n1, c, par, nxt);
+                    };
+                    chunk_expand(ex, R, C, hc, 0u, fn);
+                    continue;
                 }
+                const uint32_t i = (it - nh) * gs + lane_id();
+                const bool valid = lane_id() < gs && i < nq;
+                const uint32_t v = valid ? src[i] : 0u;
+                uint32_t r = 0, c = 0, beg = 0, deg = 0;
+                bool act = valid;
+                if (valid) {
+                    beg = __ldg(&R[v]);
+                    deg = __ldg(&R[v + 1u]) - beg;
+                    if (RAISE) {
+                        r = w.pc[v].x;
+                        c = atomicAnd(&w.pc[v].y, ~1u) >> 1;   // off the list: the newest colour
+                    } else {
+                        const uint32_t y = w.pc[v].y;
+                        c = y >> 1;
+                        if (lev == 0u) {   // the root of its colour?
+                            act = y == v << 1;
+                            if (act) {
+                                w.pc[v].y = y | 1u;
+                                w.smin[v] = v;   // v represents its SCC: the update folds the members in
+                            }
+                        }
+                    }
+                }
+                if (!RAISE && lev == 0u) {
+                    const unsigned m = __ballot_sync(FULL, act);
+                    if (lane_id() == 0 && m) atomicAdd(&ex.ctl->n_pivot, (unsigned long long)__popc(m));
+                    if (m == 0u) continue;
+                }
+                if (!act) deg = 0u;
+                const bool heavy = deg > HEAVY_T;
+                warp_push_chunks(v, heavy ? (deg + CH - 1u) / CH : 0u, w.H[0][par], &ex.lc(nxt)[C_FH], w.hcap, ex.ctl);
+                if (heavy) deg = 0u;
+                count_verts(ex, valid);
+                auto fn = [&](bool v0, uint32_t n0, uint32_t l0, bool v1, uint32_t n1, uint32_t l1) {
+                    const uint32_t c0 = __shfl_sync(FULL, c, l0), c1 = __shfl_sync(FULL, c, l1);
+                    if (RAISE) {
+                        const uint32_t r0 = __shfl_sync(FULL, r, l0), r1 = __shfl_sync(FULL, r, l1);
+                        peel_raise2(ex, g, w, v0, n0, r0, c0, v1, n1, r1, c1, par, nxt);
+                    } else {
+                        peel_join2(ex, g, w, v0, n0, c0, v1, n1, c1, par, nxt);
+                    }
+                };
+                count_edges(ex, lbs_walk2(beg, deg, C, fn));
+            }
+            bq_flush(1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], nullptr, nullptr, g.V, ex.ctl);
+        });
+        if (!ok) return false;
+        nq = last_count(ex, C_FQ);
+        nh = last_count(ex, C_FH);
+        if (nq + nh == 0u) return true;
+    }
+}
+
+// Peel end: vertices that reach their root are its SCC; the rest keep their
+// colour as range, take their own id as colour and form the next live list.
+template <class Ex>
+__device__ bool ph_peel_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
+{
+    return run_pass(ex, PH_PEEL_UPDATE, [&](unsigned, unsigned nxt) {
+        for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
+            uint32_t v[4], y[4];
+            bool ok[4];
+            load_list4(src, base + 4u * lane_id(), v, ok);
+#pragma unroll
+            for (int j = 0; j < 4; j++) y[j] = ok[j] ? w.pc[v[j]].y : 0u;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const bool scc = ok[j] && (y[j] & 1u), surv = ok[j] && !scc;
+                const uint32_t c = y[j] >> 1;
+                if (scc) {
+                    w.pc[v[j]] = make_uint2(FULL, FULL);
+                    w.st[v[j]] = DEAD;
+                    w.label[v[j]] = c;
+                }
+                if (surv) w.pc[v[j]] = make_uint2(c, (v[j] << 1) | 1u);
                 smin_fold(scc, c, v[j], w.smin);
                 bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
                 bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 17);
@@ -1058,52 +1114,6 @@ __device__ bool ph_slota_peel_update(Ex &ex, const Graph &g, const Work &w, VLis
     });
 }
 
-// Hong: compact the live list and give every live vertex its own id as
-// name (assignUniqueRange, scc_kernels.cu:477-484) before the min-label
-// propagation.
-template <class Ex>
-__device__ bool ph_compact_rename(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
-{
-    return run_pass(ex, PH_RENAME, [&](unsigned, unsigned nxt) {
-        for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
-            uint32_t v[4], s[4];
-            bool ok[4];
-            load_list4(src, base + 4u * lane_id(), v, ok);
-#pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const bool surv = s[j] != DEAD;
-                if (surv) w.st[v[j]] = v[j];
-                bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 18);
-            }
-            count_verts_n(ex, (unsigned)ok[0] + ok[1] + ok[2] + ok[3]);
-        }
-        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl);
-    });
-}
-
-// Per-range pivot bids over a list (pollForPivots, scc_kernels.cu:57-74).
-template <class Ex>
-__device__ bool ph_pivots(Ex &ex, const Graph &g, const Work &w, VList src)
-{
-    // every range is listed once, by its first bid, in Q[0][parity of this
-    // pass]: the next pass seeds the pivots from that list
-    return run_pass(ex, PH_PIVOTS, [&](unsigned, unsigned nxt) {
-        const unsigned par = ex.gl & 1u;
-        for (uint32_t base = ex.wid() * 32u; base < src.n; base += ex.nwarps() * 32u) {
-            uint32_t i = base + lane_id();
-            bool valid = i < src.n;
-            uint32_t v = valid ? src.at(i) : 0u;
-            uint32_t r = valid ? (w.st[v] & RMASK) : 0u;
-            const bool first = range_max_atomic(valid, r, valid ? pivot_key(g, v) : 0ull, w.pivkey);
-            warp_push(first, r, w.Q[0][par], &ex.lc(nxt)[C_RNG], g.V + 1u, ex.ctl, 21);
-            bq_add_edges(0, valid ? __ldg(&g.Fr[v + 1u]) - __ldg(&g.Fr[v]) : 0u);
-        }
-        bq_flush_edges(&ex.lc(nxt)[C_FE]);   // out-arcs of the live list (the residual check)
-    });
-}
-
 // ---------------------------------------------------------------------
 // drivers
 // ---------------------------------------------------------------------
@@ -1111,8 +1121,8 @@ struct Carry {
     unsigned gl;
     unsigned lsel;
     uint32_t nL;
-    uint32_t nR;    // Hong: ranges listed by the last bidding pass (in Q[0][its parity])
     uint32_t nE;    // out-arcs of the live vertices (tallied by the pass that listed them)
+    uint32_t peels; // colour peels made so far
 };
 
 enum { RUN_DONE = 0, RUN_SWITCH = 1, RUN_RESIDUAL = 2, RUN_ERROR = -1 };
@@ -1136,16 +1146,18 @@ enum { RUN_DONE = 0, RUN_SWITCH = 1, RUN_RESIDUAL = 2, RUN_ERROR = -1 };
 //   propagation (max of the local ids reachable on even peels, min on odd
 //   ones, so a chain is cut from either end) and a forward search inside
 //   each colour from its root, as scc_Coloring.cu:590-637 does, but with
-//   __syncthreads barriers between sweeps.
+//   __syncthreads barriers between sweeps and with the colours of a peel kept
+//   as ranges of the next (3,000 vertices of a chain of SCCs: 7 to 11 peels
+//   instead of 16 to 19, a third of the sweeps).
 // ---------------------------------------------------------------------
 constexpr uint32_t RES_MAX_V = 4096;
 constexpr uint32_t RES_MAX_E = 16384;
 
 __host__ __device__ __forceinline__ uint32_t res_al4(uint32_t x) { return (x + 3u) & ~3u; }
-// shared memory of the solver: gid, off, aux (u32), col (u16), flag (u8), adj (u16)
+// shared memory of the solver: gid, off, aux (u32), col, rng (u16), flag (u8), adj (u16)
 __host__ __device__ __forceinline__ uint32_t res_smem_bytes(uint32_t n, uint32_t m)
 {
-    return 4u * n + 4u * (n + 1u) + 4u * n + res_al4(2u * n) + res_al4(n) + res_al4(2u * m);
+    return 4u * n + 4u * (n + 1u) + 4u * n + 2u * res_al4(2u * n) + res_al4(n) + res_al4(2u * m);
 }
 
 // Uniform decision (same in every thread of the launch or CTA): solve the
@@ -1187,7 +1199,8 @@ __device__ __forceinline__ void block_excl_scan(uint32_t *a, uint32_t len)
 }
 
 // Passes 1 and 2 (every CTA of the policy).  On return the arcs are in
-// Q[1][(cy.gl - 1) & 1] and their number in the pass counter C_BQ.
+// Q[0][(cy.gl - 1) & 1] (the colour words lie over Q[1]) and their number in
+// the pass counter C_BQ.
 template <class Ex>
 __device__ bool res_extract(Ex &ex, const Graph &g, const Work &w, Carry &cy)
 {
@@ -1198,24 +1211,27 @@ __device__ bool res_extract(Ex &ex, const Graph &g, const Work &w, Carry &cy)
         }))
         return false;
     const bool ok = run_pass(ex, PH_RES_EXTRACT, [&](unsigned, unsigned nxt) {
-        uint32_t *eb = w.Q[1][ex.gl & 1u];
+        uint32_t *eb = w.Q[0][ex.gl & 1u];
         for (uint32_t base = ex.wid() * 32u; base < n; base += ex.nwarps() * 32u) {
             const uint32_t i = base + lane_id();
             const bool valid = i < n;
             const uint32_t v = valid ? L[i] : 0u;
             const uint32_t beg = valid ? __ldg(&g.Fr[v]) : 0u, deg = valid ? __ldg(&g.Fr[v + 1u]) - beg : 0u;
-            auto fn = [&](bool ok2, uint32_t u, uint32_t src) {
+            const uint32_t r = valid && cy.peels ? w.pc[v].x : 0u;
+            auto fn = [&](bool ok2, uint32_t u, uint32_t own) {
                 bool hit = false;
                 uint32_t e = 0;
+                const uint32_t src = __shfl_sync(FULL, i, own), rs = __shfl_sync(FULL, r, own);
                 if (ok2) {
-                    const uint32_t s = w.st[guard_id(u, g.V, ex.ctl)];
+                    u = guard_id(u, g.V, ex.ctl);
+                    const uint32_t s = w.st[u];
                     // live vertex i carries FV|BV|(i + 1); FV|BV|0 marks the first SCC's members
-                    hit = (s & (FVB | BVB)) == (FVB | BVB) && (s & RMASK) != 0u;
+                    hit = (s & (FVB | BVB)) == (FVB | BVB) && (s & RMASK) != 0u && (!cy.peels || w.pc[u].x == rs);
                     e = (src << 16) | ((s & RMASK) - 1u);
                 }
                 warp_push(hit, e, eb, &ex.lc(nxt)[C_BQ], RES_MAX_E, ex.ctl, 24);
             };
-            count_edges(ex, lbs_expand(beg, deg, i, g.Fc, fn));
+            count_edges(ex, lbs_walk(beg, deg, g.Fc, fn));
         }
     });
     cy.gl = ex.gl;
@@ -1235,18 +1251,21 @@ static __device__ __noinline__ void res_solve(const Graph &g, const Work &w, con
                           uint32_t m, Ctl *ctl, uint32_t *out = nullptr)
 {
     constexpr uint8_t ALIVE = 1, VIS = 2;
+    constexpr uint16_t RNG_DONE = 0xFFFFu;   // above every local id: matches no live vertex's range
     char *sb = reinterpret_cast<char *>(&sccb_dsmem[BQ_HDR]);
     uint32_t *gid = reinterpret_cast<uint32_t *>(sb);
     uint32_t *off = gid + n;
     uint32_t *aux = off + n + 1u;                  // fill cursor, then smallest member id per root
     uint16_t *col = reinterpret_cast<uint16_t *>(aux + n);
-    uint8_t *flag = reinterpret_cast<uint8_t *>(sb + 12u * n + 4u + res_al4(2u * n));
-    uint16_t *adj = reinterpret_cast<uint16_t *>(sb + 12u * n + 4u + res_al4(2u * n) + res_al4(n));
+    uint16_t *rng = reinterpret_cast<uint16_t *>(sb + 12u * n + 4u + res_al4(2u * n));   // colour of the last peel
+    uint8_t *flag = reinterpret_cast<uint8_t *>(sb + 12u * n + 4u + 2u * res_al4(2u * n));
+    uint16_t *adj = reinterpret_cast<uint16_t *>(sb + 12u * n + 4u + 2u * res_al4(2u * n) + res_al4(n));
     __shared__ uint32_t s_alive, s_npiv, s_peels;
     const uint32_t t = threadIdx.x, T = blockDim.x;
     for (uint32_t i = t; i < n; i += T) {
         gid[i] = L[i];
         off[i] = 0u;
+        rng[i] = 0u;
         flag[i] = ALIVE;
     }
     if (t == 0) { off[n] = 0u; s_alive = n; s_npiv = 0u; s_peels = 0u; }
@@ -1277,9 +1296,10 @@ static __device__ __noinline__ void res_solve(const Graph &g, const Work &w, con
             for (uint32_t i = t; i < n; i += T) {
                 if (!(flag[i] & ALIVE)) continue;
                 uint16_t c = col[i];
+                const uint16_t r = rng[i];
                 for (uint32_t e = off[i]; e < off[i + 1u]; e++) {
                     const uint16_t j = adj[e];
-                    if ((flag[j] & ALIVE) && col[j] > c) c = col[j];
+                    if (rng[j] == r && col[j] > c) c = col[j];
                 }
                 if (c > col[i]) { col[i] = c; ch = 1; }
             }
@@ -1307,8 +1327,12 @@ static __device__ __noinline__ void res_solve(const Graph &g, const Work &w, con
         if (failed) break;
         uint32_t done = 0, roots = 0;
         for (uint32_t i = t; i < n; i += T) {
-            if ((flag[i] & (ALIVE | VIS)) != (ALIVE | VIS)) continue;
+            if ((flag[i] & (ALIVE | VIS)) != (ALIVE | VIS)) {
+                rng[i] = (flag[i] & ALIVE) ? col[i] : RNG_DONE;
+                continue;
+            }
             const uint32_t r = up ? col[i] : n - 1u - col[i];
+            rng[i] = RNG_DONE;
             atomicMin(&aux[r], gid[i]);
             col[i] = (uint16_t)r;   // the root, from here on
             flag[i] = 0;
@@ -1354,7 +1378,7 @@ __device__ int residual(Ex &ex, const Graph &g, const Work &w, Carry &cy)
 {
     if (!res_extract(ex, g, w, cy)) return RUN_ERROR;
     if (Ex::grid) return RUN_RESIDUAL;
-    res_solve(g, w, w.L[cy.lsel], cy.nL, w.Q[1][(cy.gl - 1u) & 1u], last_count(ex, C_BQ), ex.ctl);
+    res_solve(g, w, w.L[cy.lsel], cy.nL, w.Q[0][(cy.gl - 1u) & 1u], last_count(ex, C_BQ), ex.ctl);
     res_trace(ex.ctl, ex.gl, cy.nL);
     ex.gl++;
     cy.gl = ex.gl;
@@ -1362,24 +1386,27 @@ __device__ int residual(Ex &ex, const Graph &g, const Work &w, Carry &cy)
     return ex.sync() ? RUN_DONE : RUN_ERROR;
 }
 
-// Hong main loop (scc_WCC.cu:851-930): per-range pivots, FW-BW, update,
-// until no vertex is left.  Entry: live list L[lsel] with nL entries and
-// the pivot bids of their ranges already in pivkey.
+// Colour peels until no vertex is left.  Entry: live list L[lsel] with nL
+// entries, nE out-arcs, their ranges in the state words.
 template <class Ex>
-__device__ int hong_loop(Ex &ex, const Graph &g, const Work &w, Carry &cy, uint32_t tail_n)
+__device__ int peel_loop(Ex &ex, const Graph &g, const Work &w, Carry &cy, uint32_t tail_n)
 {
     while (cy.nL > 0u) {
         if (res_fits<Ex>(g, w, cy)) return residual(ex, g, w, cy);
         if (Ex::grid && cy.nL <= tail_n) { cy.gl = ex.gl; return RUN_SWITCH; }
         if (ex.leader()) ex.ctl->outer++;
+        if (cy.peels == 0u && !ph_peel_init(ex, g, w)) return RUN_ERROR;
         const VList L{w.L[cy.lsel], cy.nL, 0u};
-        const VList R{w.Q[0][(ex.gl & 1u) ^ 1u], cy.nR, 0u};   // written by the previous pass
-        if (!ph_bfs(ex, g, w, R, SeedRanges{}, true, -1, L)) return RUN_ERROR;
-        if (!ph_hong_update(ex, g, w, L, w.L[cy.lsel ^ 1u], false, true)) return RUN_ERROR;
+        const bool odd = (cy.peels & 1u) != 0u;
+        const uint32_t *R0 = odd ? g.Br : g.Fr, *C0 = odd ? g.Bc : g.Fc;
+        const uint32_t *R1 = odd ? g.Fr : g.Br, *C1 = odd ? g.Fc : g.Bc;
+        if (!ph_peel_spread<true>(ex, g, w, L, R0, C0)) return RUN_ERROR;
+        if (!ph_peel_spread<false>(ex, g, w, L, R1, C1)) return RUN_ERROR;
+        if (!ph_peel_update(ex, g, w, L, w.L[cy.lsel ^ 1u])) return RUN_ERROR;
         cy.nL = last_count(ex, C_LIST);
-        cy.nR = last_count(ex, C_RNG);
         cy.nE = last_count(ex, C_FE);
         cy.lsel ^= 1u;
+        cy.peels++;
         cy.gl = ex.gl;
     }
     return RUN_DONE;
@@ -1431,12 +1458,12 @@ template <class Ex>
 __device__ bool first_fwbw(Ex &ex, const Graph &g, const Work &w, int lw, VList scope, VList *last = nullptr)
 {
     const unsigned long long k = vld64(&w.pivkey[0]);
-    const uint32_t p = k ? key_vertex(k) : 0u;
-    return ph_bfs(ex, g, w, VList{nullptr, k ? 1u : 0u, p}, SeedOne{p}, true, lw, scope, last);
+    if (k == 0ull) return true;   // no live vertex
+    return ph_bfs(ex, g, w, key_vertex(k), lw, scope, last);
 }
 
 // vHong / wHong up to the main loop (scc_WCC.cu:573-848): trim1*, first
-// pivot, FW-BW, update, trim1*, trim2, trim1*, "WCC", first per-range pivots.
+// pivot, FW-BW, update, trim1*, trim2, trim1*, live list of what is left.
 template <class Ex>
 __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t2, int lw, Carry &cy)
 {
@@ -1449,18 +1476,16 @@ __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t
         scope = VList{w.L[0], last_count(ex, C_LIST), 0u};
     }
     if (!first_fwbw(ex, g, w, lw, scope)) return RUN_ERROR;
-    if (!ph_hong_update(ex, g, w, scope, w.L[1], true, false)) return RUN_ERROR;
+    if (!ph_hong_update(ex, g, w, scope, w.L[1])) return RUN_ERROR;
     const VList L1{w.L[1], last_count(ex, C_LIST), 0u};
+    cy.gl = ex.gl;
+    if (L1.n == 0u) return RUN_DONE;   // every vertex is trimmed or in the first SCC
     if (t1 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
     if (t2 && !ph_trim2(ex, g, w, L1)) return RUN_ERROR;
     if (t1 && t2 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
-    if (!ph_compact_rename(ex, g, w, L1, w.L[0])) return RUN_ERROR;
+    if (!ph_compact(ex, g, w, L1, w.L[0])) return RUN_ERROR;
     cy.lsel = 0u;
     cy.nL = last_count(ex, C_LIST);
-    const VList L{w.L[0], cy.nL, 0u};
-    if (!ph_propagate<false>(ex, g, w, L)) return RUN_ERROR;
-    if (!ph_pivots(ex, g, w, L)) return RUN_ERROR;
-    cy.nR = last_count(ex, C_RNG);
     cy.nE = last_count(ex, C_FE);
     cy.gl = ex.gl;
     return RUN_DONE;
@@ -1493,27 +1518,6 @@ __device__ int slota_front(Ex &ex, const Graph &g, const Work &w, bool t1, int l
     cy.nL = last_count(ex, C_LIST);
     cy.nE = last_count(ex, C_FE);
     cy.gl = ex.gl;
-    return RUN_DONE;
-}
-
-// Colouring peels (scc_Coloring.cu:590-637): max-colour propagation, roots
-// colour == id, forward reachability inside the colour, update.
-template <class Ex>
-__device__ int slota_peels(Ex &ex, const Graph &g, const Work &w, Carry &cy, uint32_t tail_n)
-{
-    while (cy.nL > 0u) {
-        if (res_fits<Ex>(g, w, cy)) return residual(ex, g, w, cy);
-        if (Ex::grid && cy.nL <= tail_n) { cy.gl = ex.gl; return RUN_SWITCH; }
-        if (ex.leader()) ex.ctl->outer++;
-        const VList L{w.L[cy.lsel], cy.nL, 0u};
-        if (!ph_propagate<true>(ex, g, w, L)) return RUN_ERROR;
-        if (!ph_bfs(ex, g, w, L, SeedRoot{}, false, -1, L)) return RUN_ERROR;
-        if (!ph_slota_peel_update(ex, g, w, L, w.L[cy.lsel ^ 1u])) return RUN_ERROR;
-        cy.nL = last_count(ex, C_LIST);
-        cy.nE = last_count(ex, C_FE);
-        cy.lsel ^= 1u;
-        cy.gl = ex.gl;
-    }
     return RUN_DONE;
 }
 

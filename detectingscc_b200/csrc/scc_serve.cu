@@ -161,7 +161,7 @@ Caps job_caps(const scc_server *s, const Job &j, const Lane *L, bool exact)
     c.E = g(L->capE, std::max<size_t>(j.sumE, 4));
     c.N = g(L->capN, j.reqs.size());
     // one scratch slice per CTA, or per cluster for a large graph
-    const size_t per = carve_work(nullptr, j.maxV, j.maxE, true, nullptr);
+    const size_t per = carve_work(nullptr, j.maxV, j.maxE, nullptr);
     const size_t slices = j.large ? 1 : job_ctas(s, j);
     c.S = g(L->capScratch, per * slices);
     return c;
@@ -300,7 +300,7 @@ int run_job(scc_server *s, Lane *L, Job &j, double t_start, std::vector<char> &a
     j.nbig = nbig;
     const uint32_t ncta = job_ctas(s, j);
     BatchParams p{L->dgraphs, L->dorder, n, L->dFr, L->dFc, L->dBr, L->dBc, 0u, L->hout, L->hres, L->scratch,
-                  (unsigned long long)carve_work(nullptr, j.maxV, j.maxE, true, nullptr), L->dnext, nbig, nullptr,
+                  (unsigned long long)carve_work(nullptr, j.maxV, j.maxE, nullptr), L->dnext, nbig, nullptr,
                   j.large ? (uint32_t)cluster : 1u, L->hdone, s->cfg.qcap, 2u, (s->cfg.flags & SCC_FLAG_TRIM1) ? 1 : 0,
                   (s->cfg.flags & SCC_FLAG_TRIM2) ? 1 : 0, lw_of(s->cfg.algo, s->cfg.warp_width),
                   4000ull * 1000000ull, 0u, 0u};

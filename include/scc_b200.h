@@ -192,7 +192,7 @@ const char *scc_version(void);
  * front by another allocator (a framework's caching pool, a serving process
  * with a fixed budget), or a plugin whose host forbids allocations outside
  * its own pool.  Runs the single-CTA SCC kernel on a scratch area that is a
- * static __device__ array inside the library (about 1.2 MiB, held by every
+ * static __device__ array inside the library (about 0.7 MiB, held by every
  * GPU that loads the library until the process exits); the caller passes
  * device CSR arrays (SCC_FLAG_DEVICE is required) and a device buffer of V
  * labels.  Graphs above SCC_NOALLOC_MAX_VERTICES / SCC_NOALLOC_MAX_EDGES
