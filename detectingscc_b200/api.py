@@ -102,10 +102,9 @@ class Engine:
     def set_tuning(self, key: str, value: int) -> None:
         N.check(self._lib.scc_set_tuning(self._h, key.encode(), int(value)), f"scc_set_tuning({key})")
 
-    PHASES = {1: "init", 2: "trim1_once", 3: "trim1_apply", 4: "trim1_fix", 5: "trim2", 6: "trim2_apply",
-              7: "first_pivot", 8: "bfs0", 9: "bfs", 10: "prop", 11: "hong_update", 12: "slota_first_update",
-              13: "peel_update", 14: "compact", 15: "peel_scc", 16: "bfs_pull", 17: "peel_init",
-              18: "res_tag", 19: "res_extract", 20: "res_solve"}
+    PHASES = {1: "init", 4: "trim1_fix", 5: "trim2", 6: "trim2_apply", 7: "first_pivot", 8: "bfs0", 9: "bfs",
+              10: "prop", 11: "first_update", 13: "peel_update", 14: "compact", 15: "peel_scc", 16: "bfs_pull",
+              17: "peel_init", 18: "res_tag", 19: "res_extract", 20: "res_solve"}
 
     def trace(self):
         """Per-pass (phase, microseconds, items pushed) of the last run (needs set_tuning('trace', n))."""

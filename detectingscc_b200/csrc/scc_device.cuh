@@ -1,14 +1,17 @@
 // Device-side building blocks of the B200 SCC engine.
 //
-// Vertex state is one 32-bit word per vertex (st[v]):
-//   bits  0..29  range name (FW-BW subproblem, Hong) or colour (Slota);
-//                0x3FFFFFFF marks a vertex whose SCC is already known
-//                (the reference's rangeSet tag, include/scc.h:36-37)
-//   bit   30     forward-visited  (FV, include/scc.h:24)
-//   bit   31     backward-visited (BV, include/scc.h:26)
-// so one gather per adjacency entry tells whether the neighbour is live, in
-// the same subproblem and unvisited.  The reference keeps uint8 tags plus a
-// uint32 range and reads both per edge (scc_kernels.cu:374-377).
+// Vertex state is half a byte per vertex, eight vertices to a word (nb):
+//   bit 0  NL  live: its SCC is not known (the reference's rangeSet tag,
+//              include/scc.h:36-37, inverted)
+//   bit 1  NF  forward-visited  (FV, include/scc.h:24)
+//   bit 2  NB  backward-visited (BV, include/scc.h:26)
+//   bit 3  NQ  trimmed after the init pass (its label is written), or, on a
+//              live vertex, in the residual
+// Neither NL nor NQ: a vertex that the init pass trimmed.  The first search runs in one
+// range, so one gather per adjacency entry tells whether the neighbour is
+// live and unvisited; afterwards the three low bits are the vertex's range.
+// The reference keeps uint8 tags plus a uint32 range and reads both per edge
+// (scc_kernels.cu:374-377).
 //
 // Every phase is written once against an execution policy:
 //   GridExec   all CTAs of a cooperative (co-resident) launch; passes end in
@@ -22,12 +25,11 @@
 
 namespace sccb {
 
-constexpr uint32_t RMASK = 0x3FFFFFFFu;
-constexpr uint32_t DEAD = 0x3FFFFFFFu;
-constexpr uint32_t FVB = 0x40000000u;
-constexpr uint32_t BVB = 0x80000000u;
+constexpr uint32_t NL = 1u, NF = 2u, NB = 4u, NQ = 8u;
+constexpr uint32_t NCLASS = NL | NF | NB;
+constexpr uint32_t NIBS = 0x11111111u;    // bit 0 of every nibble of a word
 constexpr uint32_t FULL = 0xFFFFFFFFu;
-constexpr uint32_t MAX_V = 0x0FFFFFFEu;   // ids fit a state word's range bits and a colour word
+constexpr uint32_t MAX_V = 0x0FFFFFFEu;   // ids fit a colour word beside its flag
 // label[v] with this bit set holds v's canonical label itself (the low
 // bits): a vertex that is its own SCC (trim-1, trim-2, small residual SCCs)
 // needs no smin entry and no gather when the labels are written out.
@@ -66,8 +68,7 @@ struct __align__(128) Ctl {
     unsigned long long *trace;                     // optional: 2 words per pass
     unsigned trace_cap;
     unsigned labels_done;                          // the SCC kernel wrote the canonical labels itself
-    unsigned first_min;                            // smallest member of the first pivot's SCC when its members
-                                                   // keep the FV|BV mark (lazy Slota update); ~0 before
+    unsigned first_min;                            // smallest member of the first pivot's SCC; ~0 before
 };
 
 // A control block reset on the device (k_canon_write), as the host would
@@ -83,8 +84,8 @@ struct CtlReset {
 
 // Phase ids recorded in the pass trace.
 enum {
-    PH_INIT = 1, PH_TRIM1_ONCE = 2, PH_TRIM1_APPLY = 3, PH_TRIM1_FIX = 4, PH_TRIM2 = 5, PH_TRIM2_APPLY = 6,
-    PH_FIRST_PIVOT = 7, PH_BFS0 = 8, PH_BFS = 9, PH_PROP = 10, PH_HONG_UPDATE = 11, PH_SLOTA_FIRST_UPDATE = 12,
+    PH_INIT = 1, PH_TRIM1_FIX = 4, PH_TRIM2 = 5, PH_TRIM2_APPLY = 6,
+    PH_FIRST_PIVOT = 7, PH_BFS0 = 8, PH_BFS = 9, PH_PROP = 10, PH_FIRST_UPDATE = 11,
     PH_PEEL_UPDATE = 13, PH_COMPACT = 14, PH_PEEL_SCC = 15, PH_BFS_PULL = 16, PH_PEEL_INIT = 17,
     PH_RES_TAG = 18, PH_RES_EXTRACT = 19, PH_RES_SOLVE = 20
 };
@@ -112,16 +113,17 @@ __device__ __forceinline__ void load_off5(const uint32_t *__restrict__ R, uint32
 }
 
 struct Work {
-    uint32_t *st, *label, *stamp;
+    uint32_t *nb;               // vertex states: nibble v & 7 of word v >> 3
+    uint32_t *st;               // trim-1 stamps, then the local numbers of the residual's vertices
+    uint32_t *label;            // of vertices whose SCC is found after the first search, or trimmed after init
     uint32_t *smin;             // smin[r] = smallest member id of the SCC represented by r; set to r
                                 // when r becomes a representative (its seed pass), then folded
     uint32_t *L[2];
-    uint32_t *S[2];             // whole-GPU path: lists of the shrinking bottom-up scope (nullptr elsewhere)
     uint32_t *Q[2][2];          // [direction][parity]
     uint2 *H[2][2];             // heavy chunks (vertex, chunk) [direction][parity]
     uint32_t hcap;
     uint2 *pc;                  // colour peels: (range, colour word) per vertex, over Q[1][0] and Q[1][1]
-    unsigned long long *pivkey; // the first pivot's key
+    unsigned long long *pivkey; // the first pivot's key: over init's live vertices, over the trimmed graph's
     Ctl *ctl;
     uint32_t qcap;              // entries per CTA staging queue (dynamic shared memory)
     uint32_t bu_k;              // bottom-up BFS step when frontier edges > bu_k * scope vertices (0 = never)
@@ -130,6 +132,9 @@ struct Work {
 };
 
 constexpr uint32_t PULL_LANE = 32;   // Work::pull_lane of the batched and no-allocation paths
+
+// Bytes of the nibble array (words 0 .. V / 8).
+__host__ __device__ constexpr size_t nib_bytes(size_t V) { return ((V / 8 + 1) * 4 + 255) / 256 * 256; }
 
 // Carve the work arrays for a graph of V vertices and E edges out of `base`
 // (nullptr: only count).  Returns the bytes used.  Same layout on host and
@@ -140,44 +145,72 @@ __host__ __device__ inline size_t carve_work(char *base, uint32_t V, uint32_t E,
     const size_t n1 = (size_t)V + 1;
     const size_t hcap = (size_t)E / CH + (size_t)E / HEAVY_T + 64;
     const size_t va = (n1 * 4 + 255) / 256 * 256;       // one vertex array
+    const size_t na = nib_bytes(V);
     const size_t ha = (hcap * 8 + 255) / 256 * 256;     // one chunk queue
-    const size_t pa = 256;                              // the pivot word
+    const size_t pa = 256;                              // the pivot words
     const size_t ca = (sizeof(Ctl) + 255) / 256 * 256;
     if (w && base) {
         w->st = (uint32_t *)(base);
         w->label = (uint32_t *)(base + va);
-        w->stamp = (uint32_t *)(base + 2 * va);
-        w->smin = (uint32_t *)(base + 3 * va);
-        w->L[0] = (uint32_t *)(base + 4 * va);
-        w->L[1] = (uint32_t *)(base + 5 * va);
-        w->S[0] = w->S[1] = nullptr;
-        w->Q[0][0] = (uint32_t *)(base + 6 * va);
-        w->Q[0][1] = (uint32_t *)(base + 7 * va);
-        w->Q[1][0] = (uint32_t *)(base + 8 * va);
-        w->Q[1][1] = (uint32_t *)(base + 9 * va);
+        w->smin = (uint32_t *)(base + 2 * va);
+        w->L[0] = (uint32_t *)(base + 3 * va);
+        w->L[1] = (uint32_t *)(base + 4 * va);
+        w->Q[0][0] = (uint32_t *)(base + 5 * va);
+        w->Q[0][1] = (uint32_t *)(base + 6 * va);
+        w->Q[1][0] = (uint32_t *)(base + 7 * va);
+        w->Q[1][1] = (uint32_t *)(base + 8 * va);
         w->pc = (uint2 *)w->Q[1][0];
-        w->H[0][0] = (uint2 *)(base + 10 * va);
-        w->H[0][1] = (uint2 *)(base + 10 * va + ha);
-        w->H[1][0] = (uint2 *)(base + 10 * va + 2 * ha);
-        w->H[1][1] = (uint2 *)(base + 10 * va + 3 * ha);
+        char *h = base + 9 * va;
+        w->nb = (uint32_t *)h;
+        h += na;
+        w->H[0][0] = (uint2 *)(h);
+        w->H[0][1] = (uint2 *)(h + ha);
+        w->H[1][0] = (uint2 *)(h + 2 * ha);
+        w->H[1][1] = (uint2 *)(h + 3 * ha);
         w->hcap = (uint32_t)hcap;
-        w->pivkey = (unsigned long long *)(base + 10 * va + 4 * ha);
-        w->ctl = (Ctl *)(base + 10 * va + 4 * ha + pa);
+        w->pivkey = (unsigned long long *)(h + 4 * ha);
+        w->ctl = (Ctl *)(h + 4 * ha + pa);
     }
-    return 10 * va + 4 * ha + pa + ca;
+    return 9 * va + na + 4 * ha + pa + ca;
 }
 
 // Dynamic shared memory of the SCC kernels: BQ_HDR control words, then the
-// staging queues (at most NBQ: two frontier queues, and on the whole-GPU
-// kernel a third one for the shrinking bottom-up scope), each split into
-// one slice of qcap entries per warp of the CTA: (BQ_HDR + queues * warps *
-// qcap) words.
-constexpr unsigned NBQ = 3;
+// two staging queues, each split into one slice of qcap entries per warp of
+// the CTA; the whole-GPU kernel has room for a third, for the residual
+// solver, which takes all of it.
+constexpr unsigned NBQ = 2;
 constexpr unsigned BQ_WARPS = 32;                       // at most 1024 threads per CTA
 constexpr unsigned BQ_CNT = 16;                         // per-warp fill counts [NBQ][BQ_WARPS]
 constexpr unsigned BQ_PRE = BQ_CNT + NBQ * BQ_WARPS;    // per-warp flush offsets [NBQ][BQ_WARPS]
 constexpr unsigned BQ_HDR = BQ_PRE + NBQ * BQ_WARPS;
 extern __shared__ uint32_t sccb_dsmem[];
+
+__device__ __forceinline__ uint32_t nib_of(const uint32_t *nb, uint32_t v) { return (nb[v >> 3] >> (4u * (v & 7u))) & 15u; }
+// Sets bits of v's nibble; the nibble before.
+__device__ __forceinline__ uint32_t nib_or(uint32_t *nb, uint32_t v, uint32_t bits)
+{
+    const uint32_t sh = 4u * (v & 7u);
+    return (atomicOr(&nb[v >> 3], bits << sh) >> sh) & 15u;
+}
+// Reads *p into L1 without waiting for it.
+__device__ __forceinline__ void prime_l1(const uint32_t *p)
+{
+    uint32_t x;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(x) : "l"(p));
+}
+// Canonical label of v, or the vertex whose smin entry holds it: by its
+// nibble v is its own SCC (trimmed by init), a member of the first pivot's
+// SCC, or has its label written.
+__device__ __forceinline__ uint32_t nib_label(uint32_t s, uint32_t v, uint32_t first_min, const uint32_t *label)
+{
+    return (s & (NL | NQ)) == 0u ? LBL_SELF | v : (s & NCLASS) == NCLASS ? LBL_SELF | first_min : label[v];
+}
+// v's SCC is known and its label written.
+__device__ __forceinline__ void nib_kill(uint32_t *nb, uint32_t v)
+{
+    atomicOr(&nb[v >> 3], NQ << (4u * (v & 7u)));
+    atomicAnd(&nb[v >> 3], ~(NL << (4u * (v & 7u))));
+}
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 __device__ __forceinline__ unsigned long long gtimer()
@@ -246,7 +279,7 @@ struct GridExec {
     static constexpr bool instr = INSTR;
     static constexpr bool grid = true;
     static constexpr bool cluster = false;
-    static constexpr unsigned nbq = 3;   // staging queues of the launch's shared memory
+    static constexpr unsigned nbq = 3;   // staging queues the launch's shared memory has room for
     Ctl *ctl;
     unsigned gl;        // pass counter, identical in every thread
     unsigned cap = 0;   // pass cap of the run (0: none), see run_pass
@@ -506,14 +539,10 @@ __device__ __forceinline__ void warp_push(bool pred, uint32_t val, uint32_t *q, 
 // warp with one global atomicAdd per qcap entries, and bq_flush writes the
 // rest of all slices with one global atomicAdd per CTA and pass.  This keeps
 // the global queue tail from becoming a same-address atomic hot spot.
-__device__ __forceinline__ uint32_t *cta_first_min();
 __device__ __forceinline__ void bq_init()
 {
     for (unsigned i = threadIdx.x; i < BQ_HDR; i += blockDim.x) sccb_dsmem[i] = 0u;
-    if (threadIdx.x == 0) {
-        *cta_first_min() = 0xFFFFFFFFu;
-        *cta_err() = 0;
-    }
+    if (threadIdx.x == 0) *cta_err() = 0;
     __syncthreads();
 }
 
@@ -544,18 +573,82 @@ __device__ __forceinline__ void bq_push(unsigned qi, bool pred, uint32_t val, ui
     __syncwarp();
 }
 
-// Adds x to the CTA's frontier-edge tally of queue qi (words 12, 13).
+// K appends per lane in one go: one reading and one writing of the slice's
+// fill count instead of K (a slice too small for 32 * K entries takes them
+// one by one).
+template <int K>
+__device__ __forceinline__ void bq_pushK(unsigned qi, const bool (&pred)[K], const uint32_t (&val)[K], uint32_t qcap,
+                                         uint32_t *gq, unsigned *gcnt, uint32_t gcap, Ctl *ctl, int where)
+{
+    if (qcap < 32u * K) {
+#pragma unroll
+        for (int j = 0; j < K; j++) bq_push(qi, pred[j], val[j], qcap, gq, gcnt, gcap, ctl, where);
+        return;
+    }
+    unsigned m[K], n = 0;
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        m[j] = __ballot_sync(FULL, pred[j]);
+        n += __popc(m[j]);
+    }
+    if (n == 0u) return;
+    const unsigned lane = lane_id(), wi = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t *slice = &sccb_dsmem[BQ_HDR + (qi * (blockDim.x >> 5) + wi) * qcap];
+    unsigned *wc = &sccb_dsmem[BQ_CNT + qi * BQ_WARPS + wi];
+    unsigned cnt = *wc;
+    if (cnt + n > qcap) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(gcnt, cnt);
+        base = __shfl_sync(FULL, base, 0);
+        for (unsigned i = lane; i < cnt; i += 32u) {
+            if (base + i < gcap) gq[base + i] = slice[i];
+            else set_error(ctl, E_OVERFLOW, where);
+        }
+        __syncwarp();
+        cnt = 0;
+    }
+    unsigned at = cnt;
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        if (pred[j]) slice[at + __popc(m[j] & lt)] = val[j];
+        at += __popc(m[j]);
+    }
+    __syncwarp();
+    if (lane == 0) *wc = at;
+    __syncwarp();
+}
+
+// Takes up to 32 of the newest entries off the warp's slice of queue qi, if
+// it holds least to most of them; lane l < the result gets one in val.
+__device__ __forceinline__ unsigned bq_pop(unsigned qi, uint32_t qcap, uint32_t least, uint32_t most,
+                                           uint32_t &val)
+{
+    const unsigned wi = threadIdx.x >> 5, lane = lane_id();
+    const uint32_t *slice = &sccb_dsmem[BQ_HDR + (qi * (blockDim.x >> 5) + wi) * qcap];
+    unsigned *wc = &sccb_dsmem[BQ_CNT + qi * BQ_WARPS + wi];
+    const unsigned cnt = *wc;
+    if (cnt < least || cnt > most) return 0u;
+    const unsigned n = min(cnt, 32u);
+    val = lane < n ? slice[cnt - n + lane] : 0u;
+    __syncwarp();
+    if (lane == 0) *wc = cnt - n;
+    __syncwarp();
+    return n;
+}
+
+// Adds x to the CTA's tally qi (words 12 .. 14): the frontier edges of queues
+// 0 and 1, and the scope left by a bottom-up step.
 __device__ __forceinline__ void bq_add_edges(unsigned qi, unsigned x)
 {
     x = __reduce_add_sync(FULL, x);
     if (lane_id() == 0 && x) atomicAdd(&sccb_dsmem[12 + qi], x);
 }
 
-// Called by every thread of the CTA at the end of a pass.  ecnt0 / ecnt1
-// (optional) receive the CTA's frontier-edge tallies.
+// Called by every thread of the CTA at the end of a pass.  ecnt0, ecnt1 and
+// scnt (optional) receive the CTA's tallies.
 __device__ __forceinline__ void bq_flush(unsigned nq, uint32_t qcap, uint32_t *gq0, unsigned *gcnt0, uint32_t *gq1,
                                          unsigned *gcnt1, uint32_t gcap, Ctl *ctl, unsigned *ecnt0 = nullptr,
-                                         unsigned *ecnt1 = nullptr, uint32_t *gq2 = nullptr, unsigned *gcnt2 = nullptr)
+                                         unsigned *ecnt1 = nullptr, unsigned *scnt = nullptr)
 {
     __syncthreads();
     const unsigned nw = blockDim.x >> 5;
@@ -574,15 +667,19 @@ __device__ __forceinline__ void bq_flush(unsigned nq, uint32_t qcap, uint32_t *g
         if (ln < nw) sccb_dsmem[BQ_PRE + qi * BQ_WARPS + ln] = incl - c;
         const unsigned total = __shfl_sync(FULL, incl, 31);
         if (ln == 0) {
-            sccb_dsmem[8 + qi] = total ? atomicAdd(qi == 2 ? gcnt2 : qi ? gcnt1 : gcnt0, total) : 0u;
-            unsigned *ec = qi == 2 ? nullptr : qi ? ecnt1 : ecnt0;
+            sccb_dsmem[8 + qi] = total ? atomicAdd(qi ? gcnt1 : gcnt0, total) : 0u;
+            unsigned *ec = qi ? ecnt1 : ecnt0;
             if (ec && sccb_dsmem[12 + qi]) atomicAdd(ec, sccb_dsmem[12 + qi]);
             sccb_dsmem[12 + qi] = 0u;
+            if (qi == 0) {
+                if (scnt && sccb_dsmem[14]) atomicAdd(scnt, sccb_dsmem[14]);
+                sccb_dsmem[14] = 0u;
+            }
         }
     }
     __syncthreads();
     for (unsigned qi = 0; qi < nq; qi++) {
-        uint32_t *gq = qi == 2 ? gq2 : qi ? gq1 : gq0;
+        uint32_t *gq = qi ? gq1 : gq0;
         const unsigned cnt = sccb_dsmem[BQ_CNT + qi * BQ_WARPS + wi];
         const unsigned base = sccb_dsmem[8 + qi] + sccb_dsmem[BQ_PRE + qi * BQ_WARPS + wi];
         const uint32_t *slice = &sccb_dsmem[BQ_HDR + (qi * nw + wi) * qcap];
@@ -592,42 +689,6 @@ __device__ __forceinline__ void bq_flush(unsigned nq, uint32_t qcap, uint32_t *g
         }
         __syncwarp();
         if (lane_id() == 0) sccb_dsmem[BQ_CNT + qi * BQ_WARPS + wi] = 0u;
-    }
-}
-
-// Per-CTA minimum of the vertices whose second visited bit (FV then BV or
-// BV then FV) was set by this CTA: the members of the first pivot's SCC
-// during the first search.  Cleared at kernel entry (bq_init).
-__device__ __forceinline__ uint32_t *cta_first_min()
-{
-    __shared__ uint32_t s_first_min;
-    return &s_first_min;
-}
-// old: the state word before an atomicOr of `bits`: v if that atomicOr
-// completed both visited bits, else ~0.
-__device__ __forceinline__ uint32_t completed(uint32_t old, uint32_t bits, uint32_t v)
-{
-    return ((old & (FVB | BVB)) != (FVB | BVB) && ((old | bits) & (FVB | BVB)) == (FVB | BVB)) ? v : 0xFFFFFFFFu;
-}
-// Folds the warp's smallest completed vertex into the CTA's minimum: one
-// warp reduction, and a shared-memory atomic only when it lowers the CTA's
-// current value (the first SCC's smallest member is found early, so almost
-// every call ends at the comparison).  All 32 lanes call.
-__device__ __forceinline__ void fold_completed(uint32_t cand)
-{
-    const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, cand);
-    if ((threadIdx.x & 31u) == 0u && m < *(volatile uint32_t *)cta_first_min()) atomicMin(cta_first_min(), m);
-}
-
-// Adds the CTA's frontier-edge tally of queue 0 (word 12) to *ecnt and
-// clears it: the end of a pass that tallies without staging queues.
-// Called by every thread of the CTA.
-__device__ __forceinline__ void bq_flush_edges(unsigned *ecnt)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (sccb_dsmem[12]) atomicAdd(ecnt, sccb_dsmem[12]);
-        sccb_dsmem[12] = 0u;
     }
 }
 
@@ -724,6 +785,33 @@ __device__ __forceinline__ unsigned lbs_walk2(uint32_t beg, uint32_t deg, const 
     return total;
 }
 
+// Same walk, four entries per lane per step: fn(valid[4], neighbour[4]).
+template <class Fn>
+__device__ __forceinline__ unsigned lbs_walk4(uint32_t beg, uint32_t deg, const uint32_t *__restrict__ C, Fn &&fn)
+{
+    const unsigned incl = warp_incl_scan(deg), total = __shfl_sync(FULL, incl, 31), excl = incl - deg;
+    const uint32_t at = beg - excl;   // entry e of a list lies at C[at of its owner + e]
+    for (unsigned base = 0; base < total; base += 128u) {
+        bool ok[4];
+        uint32_t n[4];
+#pragma unroll
+        for (unsigned j = 0; j < 4u; j++) {
+            const unsigned e = base + 32u * j + lane_id();
+            unsigned lo = 0;
+#pragma unroll
+            for (unsigned step = 16; step >= 1; step >>= 1) {
+                const unsigned x = __shfl_sync(FULL, excl, (lo + step) & 31u);
+                if (lo + step < 32u && x <= e) lo += step;
+            }
+            const uint32_t a = __shfl_sync(FULL, at, lo);
+            ok[j] = e < total;
+            n[j] = ok[j] ? __ldg(&C[a + e]) : 0u;
+        }
+        fn(ok, n);
+    }
+    return total;
+}
+
 // The same with one value per owner: fn(v0, n0, aux0, v1, n1, aux1).
 template <class Fn>
 __device__ __forceinline__ unsigned lbs_expand2(uint32_t beg, uint32_t deg, uint32_t aux,
@@ -753,28 +841,10 @@ __device__ __forceinline__ void smin_fold(bool valid, uint32_t rep, uint32_t v, 
     if (valid && lane_id() == (unsigned)(__ffs(grp) - 1) && mn < vld(&smin[rep])) atomicMin(&smin[rep], mn);
 }
 
-// Virtual-warp expansion: groups of W = 1 << lw lanes share one vertex and
+// Virtual-warp expansion: groups of W = 1 << lw lanes share a vertex and
 // stride over its adjacency (the reference's fwd_warp/bwd_warp schedule,
-// include/scc_kernels.h:46-105).  Returns the entries scanned by the warp.
-template <class Fn>
-__device__ __forceinline__ unsigned vw_expand(uint32_t beg, uint32_t deg, uint32_t aux, unsigned lw,
-                                              const uint32_t *__restrict__ C, Fn &&fn)
-{
-    unsigned W = 1u << lw;
-    unsigned sub = lane_id() & (W - 1u);
-    unsigned maxd = __reduce_max_sync(FULL, deg);
-    for (unsigned base = 0; base < maxd; base += W) {
-        unsigned k = base + sub;
-        bool valid = k < deg;
-        uint32_t nbr = valid ? __ldg(&C[beg + k]) : 0u;
-        fn(valid, nbr, aux);
-    }
-    unsigned own = (sub == 0u) ? deg : 0u;
-    return __reduce_add_sync(FULL, own);
-}
-
-// Virtual-warp expansion of K vertices per lane group at once (the same W
-// lanes per vertex as vw_expand): the K lists are walked in the same steps,
+// include/scc_kernels.h:46-105), K vertices per lane group at once: the K
+// lists are walked in the same steps,
 // so every lane has K gathers in flight.  fn(j, valid, nbr) per entry, in
 // pairs of j; returns the entries of the warp.
 template <int K, class Fn>
@@ -824,22 +894,6 @@ __device__ __forceinline__ void block_min_atomic(uint32_t x, uint32_t *dst)
     __syncthreads();
 }
 
-// 32-bit max over the warp, then the CTA; the CTA's thread 0 performs one
-// atomicMax.  Called by every thread of the CTA.
-__device__ __forceinline__ void block_max_atomic32(uint32_t x, uint32_t *dst)
-{
-    __shared__ uint32_t s_max[32];
-    const uint32_t m = __reduce_max_sync(FULL, x);
-    const unsigned wi = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane_id() == 0) s_max[wi] = m;
-    __syncthreads();
-    if (wi == 0) {
-        const uint32_t r = __reduce_max_sync(FULL, lane_id() < nw ? s_max[lane_id()] : 0u);
-        if (lane_id() == 0 && r > *(volatile uint32_t *)dst) atomicMax(dst, r);
-    }
-    __syncthreads();
-}
-
 // 64-bit max of a pivot key over the warp, then the CTA; the CTA's thread 0
 // performs one atomicMax.  With dst32 set, the 32-bit max of x goes to
 // dst32 in the same two barriers.  Called by every thread of the CTA.
@@ -878,12 +932,5 @@ __device__ __forceinline__ unsigned long long pivot_key(const Graph &g, uint32_t
     return ((unsigned long long)prod << 32) | (unsigned long long)(0xFFFFFFFFu - v);
 }
 __device__ __forceinline__ uint32_t key_vertex(unsigned long long k) { return 0xFFFFFFFFu - (uint32_t)k; }
-
-// Ranges after the first FW-BW split: 1 neither, 2 forward only, 3 backward
-// only (the reference's 3*range + FV + 2*BV, scc_kernels.cu:138, for range 0).
-__device__ __forceinline__ uint32_t split_class(uint32_t s)
-{
-    return 1u + ((s & FVB) ? 1u : 0u) + ((s & BVB) ? 2u : 0u);
-}
 
 }  // namespace sccb

@@ -34,7 +34,7 @@ struct Params {
 };
 
 // Canonical labels of vertices tid+1, tid+1+n, ...: every vertex takes the
-// smallest member id of its SCC, which the update passes fold into
+// smallest member id of its SCC, which the peel updates fold into
 // smin[representative] (or label[v] holds it itself, LBL_SELF).  Runs after the last pass barrier, so label and
 // smin are final.  Four vertices per thread and round: their label loads,
 // then their smin gathers, are issued back to back, so a thread waits on
@@ -44,25 +44,20 @@ struct Params {
 // non-coherent read-only path.
 constexpr uint32_t LABEL_UNROLL = 4;
 
-// A vertex whose state still carries both visited bits with range 0 is a
-// member of the first pivot's SCC left marked by the lazy Slota update; its
-// label is first_min.
-// SKIP_RESIDUAL: vertices still carrying the residual solver's tag
-// (FV|BV|(i+1)) are left out; the solver writes theirs.
+// SKIP_RESIDUAL: vertices in the residual are left out; the solver writes
+// theirs.
 template <bool SKIP_RESIDUAL = false>
-__device__ __forceinline__ void canon_labels(const uint32_t *label, const uint32_t *smin, const uint32_t *st,
+__device__ __forceinline__ void canon_labels(const uint32_t *label, const uint32_t *smin, const uint32_t *nb,
                                              uint32_t first_min, uint32_t *out, uint32_t V, uint32_t tid, uint32_t n)
 {
     for (uint32_t v0 = tid + 1u; v0 <= V; v0 += LABEL_UNROLL * n) {
-        uint32_t l[LABEL_UNROLL];
-        bool skip[LABEL_UNROLL];
+        uint32_t l[LABEL_UNROLL], s[LABEL_UNROLL];
+#pragma unroll
+        for (uint32_t j = 0; j < LABEL_UNROLL; ++j) s[j] = v0 + j * n <= V ? nib_of(nb, v0 + j * n) : 0u;
 #pragma unroll
         for (uint32_t j = 0; j < LABEL_UNROLL; ++j) {
             const uint32_t v = v0 + j * n;
-            l[j] = v <= V ? label[v] : 0xFFFFFFFFu;
-            const uint32_t s = v <= V ? st[v] : DEAD;
-            if (s == (FVB | BVB)) l[j] = LBL_SELF | first_min;
-            skip[j] = SKIP_RESIDUAL && (s & (FVB | BVB)) == (FVB | BVB) && (s & RMASK) != 0u;
+            l[j] = v <= V ? nib_label(s[j], v, first_min, label) : LBL_SELF;
         }
 #pragma unroll
         for (uint32_t j = 0; j < LABEL_UNROLL; ++j)
@@ -70,14 +65,14 @@ __device__ __forceinline__ void canon_labels(const uint32_t *label, const uint32
 #pragma unroll
         for (uint32_t j = 0; j < LABEL_UNROLL; ++j) {
             const uint32_t v = v0 + j * n;
-            if (v <= V && !skip[j]) out[v - 1u] = l[j];
+            if (v <= V && !(SKIP_RESIDUAL && (s[j] & (NL | NQ)) == (NL | NQ))) out[v - 1u] = l[j];
         }
     }
 }
 
 __device__ __forceinline__ void write_labels(const Work &w, uint32_t V, uint32_t *out, uint32_t tid, uint32_t n)
 {
-    canon_labels(w.label, w.smin, w.st, *(volatile const uint32_t *)&w.ctl->first_min, out, V, tid, n);
+    canon_labels(w.label, w.smin, w.nb, *(volatile const uint32_t *)&w.ctl->first_min, out, V, tid, n);
 }
 
 // ---------------------------------------------------------------------
@@ -86,7 +81,7 @@ __device__ __forceinline__ void write_labels(const Work &w, uint32_t V, uint32_t
 constexpr int GRID_THREADS = 1024;
 constexpr int BLOCK_THREADS = 1024;
 
-// queues: staging queues of the launch (3 on the whole-GPU kernel, 2 on one CTA)
+// queues: room in staging queues (3 on the whole-GPU kernel, 2 on one CTA)
 static size_t dyn_smem_bytes(uint32_t qcap, unsigned queues, int threads = 1024)
 {
     return (BQ_HDR + queues * (size_t)(threads / 32) * qcap) * sizeof(uint32_t);
@@ -108,7 +103,7 @@ __global__ void __launch_bounds__(GRID_THREADS, 1) k_scc_grid(Params p)
         // outside the residual is final here)
         if (blockIdx.x != 0) {
             if (p.out)
-                canon_labels<true>(p.w.label, p.w.smin, p.w.st, *(volatile const uint32_t *)&p.w.ctl->first_min, p.out,
+                canon_labels<true>(p.w.label, p.w.smin, p.w.nb, *(volatile const uint32_t *)&p.w.ctl->first_min, p.out,
                                    p.g.V, (blockIdx.x - 1u) * blockDim.x + threadIdx.x, (gridDim.x - 1u) * blockDim.x);
             return;
         }
@@ -166,7 +161,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) k_scc_block(Params p)
 // which the update passes fold into smin[representative].
 // Skipped when the SCC kernel already wrote them (ctl->labels_done).
 __global__ void k_canon_write(const uint32_t *__restrict__ label, const uint32_t *__restrict__ smin,
-                              const uint32_t *__restrict__ st, uint32_t *__restrict__ out, uint32_t V, const Ctl *ctl,
+                              const uint32_t *__restrict__ nb, uint32_t *__restrict__ out, uint32_t V, const Ctl *ctl,
                               CtlReset r)
 {
     if (blockIdx.x == 0 && r.next) {
@@ -179,11 +174,11 @@ __global__ void k_canon_write(const uint32_t *__restrict__ label, const uint32_t
             r.next->timeout_ns = r.timeout_ns;
             r.next->trace = r.trace;
             r.next->trace_cap = r.trace_cap;
-            if (r.pivkey) *r.pivkey = 0ull;
+            if (r.pivkey) r.pivkey[0] = r.pivkey[1] = 0ull;
         }
     }
     if (ctl && ctl->labels_done) return;
-    canon_labels(label, smin, st, ctl ? ctl->first_min : 0xFFFFFFFFu, out, V, blockIdx.x * blockDim.x + threadIdx.x,
+    canon_labels(label, smin, nb, ctl ? ctl->first_min : 0xFFFFFFFFu, out, V, blockIdx.x * blockDim.x + threadIdx.x,
                  gridDim.x * blockDim.x);
 }
 
@@ -239,7 +234,7 @@ namespace {
 
 // Offsets of the whole-graph workspace (all 256-byte aligned).
 struct WsLayout {
-    size_t st, label, stamp, smin, L0, L1, S0, S1, Q[4], H[4], piv, ctl, need, hcap;
+    size_t nb, st, label, smin, L0, L1, Q[4], H[4], piv, ctl, need, hcap;
 };
 
 WsLayout ws_layout(uint32_t V, uint32_t E)
@@ -249,12 +244,11 @@ WsLayout ws_layout(uint32_t V, uint32_t E)
     const size_t n1 = (size_t)V + 1;
     size_t need = 0;
     auto take = [&](size_t bytes) { size_t off = need; need = align_up(need + bytes, 256); return off; };
-    o.st = take(n1 * 4); o.label = take(n1 * 4); o.stamp = take(n1 * 4); o.smin = take(n1 * 4);
+    o.nb = take(nib_bytes(V)); o.st = take(n1 * 4); o.label = take(n1 * 4); o.smin = take(n1 * 4);
     o.L0 = take(n1 * 4); o.L1 = take(n1 * 4);
-    o.S0 = take(n1 * 4); o.S1 = take(n1 * 4);
     for (int i = 0; i < 4; i++) o.Q[i] = take(n1 * 4);
     for (int i = 0; i < 4; i++) o.H[i] = take(o.hcap * sizeof(uint2));
-    o.piv = take(8);
+    o.piv = take(16);
     o.ctl = take(sizeof(Ctl));
     o.need = need;
     return o;
@@ -268,7 +262,7 @@ int scc_ctx_reserve(scc_context *ctx, uint32_t V, uint32_t E)
 {
     const WsLayout o = ws_layout(V, E);
     const size_t need = o.need, hcap = o.hcap;
-    const size_t o_st = o.st, o_label = o.label, o_stamp = o.stamp, o_smin = o.smin, o_L0 = o.L0, o_L1 = o.L1;
+    const size_t o_st = o.st, o_label = o.label, o_smin = o.smin, o_L0 = o.L0, o_L1 = o.L1;
     const size_t *o_Q = o.Q, *o_H = o.H;
     const size_t o_piv = o.piv, o_ctl = o.ctl;
     if (need > ctx->ws_bytes) {
@@ -283,12 +277,10 @@ int scc_ctx_reserve(scc_context *ctx, uint32_t V, uint32_t E)
     Work &w = ctx->work;
     w.st = (uint32_t *)(b + o_st);
     w.label = (uint32_t *)(b + o_label);
-    w.stamp = (uint32_t *)(b + o_stamp);
+    w.nb = (uint32_t *)(b + o.nb);
     w.smin = (uint32_t *)(b + o_smin);
     w.L[0] = (uint32_t *)(b + o_L0);
     w.L[1] = (uint32_t *)(b + o_L1);
-    w.S[0] = (uint32_t *)(b + o.S0);
-    w.S[1] = (uint32_t *)(b + o.S1);
     w.Q[0][0] = (uint32_t *)(b + o_Q[0]);
     w.Q[0][1] = (uint32_t *)(b + o_Q[1]);
     w.Q[1][0] = (uint32_t *)(b + o_Q[2]);
@@ -576,7 +568,7 @@ static int run_impl(scc_context *ctx, const scc_csr_view *gv, int algo, uint32_t
                                  ctx->work.ctl, st, dev ? nullptr : gv->Fc);
         if (rc != SCC_OK) return rc;
     }
-    if (!piv_ready) CK(cudaMemsetAsync(ctx->work.pivkey, 0, 8, st));
+    if (!piv_ready) CK(cudaMemsetAsync(ctx->work.pivkey, 0, 16, st));
 
 
     ctx->work.qcap = ctx->qcap;
@@ -606,7 +598,7 @@ static int run_impl(scc_context *ctx, const scc_csr_view *gv, int algo, uint32_t
     launches++;
     CK(cudaEventRecord(ctx->ev[2], st));
     if (dout) {
-        k_canon_write<<<canon_ctas(V), 256, 0, st>>>(ctx->work.label, ctx->work.smin, ctx->work.st, dout, V,
+        k_canon_write<<<canon_ctas(V), 256, 0, st>>>(ctx->work.label, ctx->work.smin, ctx->work.nb, dout, V,
                                                      ctx->work.ctl, init);
         launches += 1;
         CK(cudaGetLastError());
@@ -723,7 +715,7 @@ int sccb_launch_block_path(const Graph &g, const Work &w, int t1, int t2, int lw
     void *args[] = {&p};
     cudaError_t e = cudaLaunchKernel(fn, dim3(1), dim3(BLOCK_THREADS), args, smem, st);
     if (e != cudaSuccess) return cuda_status(e);
-    k_canon_write<<<canon_ctas(g.V), 256, 0, st>>>(w.label, w.smin, w.st, dout, g.V, w.ctl, CtlReset{});
+    k_canon_write<<<canon_ctas(g.V), 256, 0, st>>>(w.label, w.smin, w.nb, dout, g.V, w.ctl, CtlReset{});
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e);
     *launches = 2;

@@ -47,12 +47,12 @@ constexpr uint32_t NOALLOC_QCAP = 512;
 constexpr size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
 // Bytes the single-CTA kernel needs for a graph of V vertices and E edges
-// (the same arrays scc_run sizes per graph: vertex state, labels, stamps,
+// (the same arrays scc_run sizes per graph: vertex states, labels, stamps,
 // two live lists, four frontier queues, four heavy-chunk queues, the pivot
 // word and the control block).
 constexpr size_t scratch_bytes(size_t V, size_t E)
 {
-    return al256((V + 1) * 4) * 10 + al256((E / CH + E / HEAVY_T + 64) * 8) * 4 + al256(8) +
+    return al256((V + 1) * 4) * 9 + nib_bytes(V) + al256((E / CH + E / HEAVY_T + 64) * 8) * 4 + al256(16) +
            al256(sizeof(Ctl));
 }
 
@@ -180,22 +180,21 @@ extern "C" int scc_run_noalloc(const scc_csr_view *gv, int algo, uint32_t flags,
     Work w{};
     w.st = (uint32_t *)take(n1 * 4);
     w.label = (uint32_t *)take(n1 * 4);
-    w.stamp = (uint32_t *)take(n1 * 4);
     w.smin = (uint32_t *)take(n1 * 4);
     w.L[0] = (uint32_t *)take(n1 * 4);
     w.L[1] = (uint32_t *)take(n1 * 4);
-    w.S[0] = w.S[1] = nullptr;   // the single-CTA kernel keeps no shrinking scope
     w.Q[0][0] = (uint32_t *)take(n1 * 4);
     w.Q[0][1] = (uint32_t *)take(n1 * 4);
     w.Q[1][0] = (uint32_t *)take(n1 * 4);
     w.Q[1][1] = (uint32_t *)take(n1 * 4);
     w.pc = (uint2 *)w.Q[1][0];   // Q[1][0] and Q[1][1] are adjacent
+    w.nb = (uint32_t *)take(nib_bytes(V));
     w.H[0][0] = (uint2 *)take(hcap * 8);
     w.H[0][1] = (uint2 *)take(hcap * 8);
     w.H[1][0] = (uint2 *)take(hcap * 8);
     w.H[1][1] = (uint2 *)take(hcap * 8);
     w.hcap = (uint32_t)hcap;
-    w.pivkey = (unsigned long long *)take(8);
+    w.pivkey = (unsigned long long *)take(16);
     w.ctl = (Ctl *)take(sizeof(Ctl));
     w.qcap = NOALLOC_QCAP;
     w.bu_k = 2;
@@ -206,7 +205,7 @@ extern "C" int scc_run_noalloc(const scc_csr_view *gv, int algo, uint32_t flags,
     Graph g{V, E, gv->Fr, gv->Fc ? gv->Fc : w.st, gv->Br, gv->Bc ? gv->Bc : w.st,
             ((((uintptr_t)gv->Fr) | ((uintptr_t)gv->Br)) & 15u) == 0u ? 1u : 0u};
     k_noalloc_ctl_init<<<1, 32, 0, st>>>(w.ctl, 4000ull * 1000000ull);
-    if (cudaMemsetAsync(w.pivkey, 0, 8, st) != cudaSuccess) {
+    if (cudaMemsetAsync(w.pivkey, 0, 16, st) != cudaSuccess) {
         cudaGetLastError();
         return SCC_ERR_CUDA;
     }

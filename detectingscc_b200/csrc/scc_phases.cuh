@@ -58,32 +58,381 @@ __device__ __forceinline__ void count_verts_n(Ex &ex, unsigned n)
     }
 }
 
-// Does v have a live neighbour in range r in (R, C)?  Early exit, as in
-// trim1 (scc_kernels.cu:197-222).  Self-loops count, as they do there.
+// Vertices a warp takes at once from a list of n (1 << item_shift): the smallest power of two
+// that still gives every warp at most one item, at most 32.  A level's time
+// is the chain of dependent accesses of its longest item, so a short list is
+// spread over all warps before lanes are filled.
 template <class Ex>
-__device__ __forceinline__ bool has_live(Ex &ex, const uint32_t *st, const uint32_t *__restrict__ R,
-                                         const uint32_t *__restrict__ C, uint32_t v, uint32_t r, uint32_t V)
+__device__ __forceinline__ uint32_t item_shift(const Ex &ex, uint32_t n)
 {
-    uint32_t e = __ldg(&R[v]), end = __ldg(&R[v + 1]);
-    bool found = false;
-    uint32_t e0 = e;
-    for (; e < end; e++) {
-        if ((st[guard_id(__ldg(&C[e]), V, ex.ctl)] & RMASK) == r) { found = true; e++; break; }
+    const uint32_t nw = ex.nwarps();
+    uint32_t s = 0;
+#pragma unroll
+    for (int i = 0; i < 5; i++) s += (n + (1u << s) - 1u) >> s > nw ? 1u : 0u;
+    return s;
+}
+template <class Ex>
+__device__ __forceinline__ uint32_t item_group(const Ex &ex, uint32_t n)
+{
+    return 1u << item_shift(ex, n);
+}
+
+// Rounds that a warp goes on for by itself at the end of its items of a
+// pass: it takes what it just appended off its own staging slice (the newest
+// 32) and expands that, while the slice holds at most local_cap entries and
+// it walked fewer than LOCAL_EDGES arcs.  A
+// search does not depend on the order its vertices are expanded in, so a
+// pass need not be one level: a high-diameter graph takes a tenth of the
+// barriers, and a vertex's neighbours are expanded while their sectors are
+// still cached.  A level-synchronous pass costs 6 to 7 us on the whole GPU
+// whatever the frontier (queue entry, offsets, arcs, state, claim, append,
+// flush, barrier), a local round 3 to 4.  701^2 grid, vHong: 125 levels in
+// 0.93 ms, now 8 passes in 0.40 ms; 50,021-vertex random graph of degree 4:
+// 13 levels in 88 us, now 2 passes in 48 us; 4096^2 grid: 163 levels in
+// 2.95 ms, now 15 passes in 2.28 ms (bound by the latency of scattered
+// sectors: DRAM and issue slots are each below 25 % busy).  Longer slices, and what is left after the last round, go
+// to the global queue and are spread over all warps by the next pass.
+// Until there is work for every warp (full) only short slices stay: a warp
+// whose slice grows fast shares it.
+constexpr uint32_t LOCAL_ROUNDS = 16, FULL_ROUNDS = 16, LOCAL_EDGES = 4096;   // of the first search
+constexpr uint32_t PEEL_ROUNDS = 8;     // of the peels
+__device__ __forceinline__ uint32_t local_cap(uint32_t qcap, bool full = false)
+{
+    return full && qcap > 256u ? qcap - 128u : min(96u, qcap / 2u);
+}
+
+// Bits 0, 4, ..., 28 of a nibble word as bits 0 .. 7.
+__device__ __forceinline__ uint32_t nib8(uint32_t m)
+{
+    m &= NIBS;
+    m = (m | m >> 3) & 0x03030303u;
+    m = (m | m >> 6) & 0x000F000Fu;
+    return (m | m >> 12) & 0xFFu;
+}
+// The live, forward- and backward-visited bits of a unit: the 32 vertices
+// 32 * u .. 32 * u + 31, four nibble words (units are whole: ph_init writes
+// the words past V as zero).
+struct NibUnit {
+    uint32_t live, fwd, bwd;
+};
+__device__ __forceinline__ NibUnit load_unit(const Work &w, bool in, uint32_t u)
+{
+    const uint4 x = in ? *reinterpret_cast<const uint4 *>(w.nb + 4u * u) : make_uint4(0u, 0u, 0u, 0u);
+    auto four = [&](int k) { return nib8(x.x >> k) | nib8(x.y >> k) << 8 | nib8(x.z >> k) << 16 | nib8(x.w >> k) << 24; };
+    return NibUnit{four(0), four(1), four(2)};
+}
+// Units a warp takes at once when about n of V vertices are marked: as many
+// as hold the 64 marks of one step of unit_walk2.
+template <class Ex>
+__device__ __forceinline__ uint32_t unit_group(const Ex &ex, uint32_t V, uint32_t n)
+{
+    const uint32_t c = (uint32_t)min(32ull, 2ull * V / max(n, 1u));
+    return max(1u, min(c, item_group(ex, V / 32u + 1u)));
+}
+
+// Walks the marked vertices (mask m of each lane's unit u), 64 at a time:
+// fn(ok[2], v[2], unit's lane[2]) is called by all lanes.  Marks are packed
+// into full lanes, so a sparse unit costs its marks, not its width.
+template <class Fn>
+__device__ __forceinline__ void unit_walk2(uint32_t u, uint32_t m, Fn &&fn)
+{
+    const unsigned c = __popc(m), incl = warp_incl_scan(c), total = __shfl_sync(FULL, incl, 31), excl = incl - c;
+    for (unsigned base = 0; base < total; base += 64u) {
+        bool ok[2];
+        uint32_t v[2];
+        unsigned own[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const unsigned e = base + 32u * (unsigned)h + lane_id();
+            unsigned lo = 0;
+#pragma unroll
+            for (unsigned step = 16; step >= 1; step >>= 1) {
+                const unsigned x = __shfl_sync(FULL, excl, (lo + step) & 31u);
+                if (lo + step < 32u && x <= e) lo += step;
+            }
+            uint32_t mo = __shfl_sync(FULL, m, lo), k = e - __shfl_sync(FULL, excl, lo), at = 0;
+            const uint32_t uo = __shfl_sync(FULL, u, lo);
+#pragma unroll
+            for (unsigned b = 16; b >= 1; b >>= 1) {   // the k-th set bit
+                const uint32_t n = __popc(mo & ((1u << b) - 1u));
+                if (k >= n) {
+                    k -= n;
+                    mo >>= b;
+                    at += b;
+                }
+            }
+            ok[h] = e < total;
+            v[h] = ok[h] ? uo * 32u + at : 0u;
+            own[h] = lo;
+        }
+        fn(ok, v, own);
     }
-    if constexpr (Ex::instr) atomicAdd(&ex.ctl->t_edges, (unsigned long long)(e - e0));
+}
+
+// Does each of the lane's four lists hold a vertex u with (nibble(u) & m) ==
+// want?  Lists 0 and 2 lie in (Br, Bc), 1 and 3 in (Fr, Fc); mr, mf are their
+// masks.  Every lane keeps its four searches in flight, two entries per step,
+// so it waits on one round of gathers for all of them; of a list longer than
+// pull_lane the lane tests the first entries (a hit is usually among them)
+// and the whole warp the rest.  Bit t of the result: list t has one.
+template <class Ex>
+__device__ __forceinline__ uint32_t find4(Ex &ex, const Graph &g, const Work &w, uint32_t (&pos)[4],
+                                          const uint32_t (&end)[4], uint32_t mr, uint32_t mf,
+                                          const uint32_t (&want)[4])
+{
+    unsigned scanned = 0;
+    uint32_t lim[4], found = 0u, on = 0u;
+    const uint32_t first = min(8u, w.pull_lane);
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        on |= end[t] > pos[t] ? 1u << t : 0u;
+        lim[t] = end[t] - pos[t] <= w.pull_lane ? end[t] : pos[t] + first;
+    }
+    const uint32_t any = on;
+    while (on) {
+        uint32_t c0[4], c1[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const uint32_t *C = (t & 1) ? g.Fc : g.Bc;
+            const bool o = (on >> t) & 1u;
+            c0[t] = o ? __ldg(&C[pos[t]]) : 0u;
+            c1[t] = o && pos[t] + 1u < end[t] ? __ldg(&C[pos[t] + 1u]) : 0u;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            if (!((on >> t) & 1u)) continue;
+            const uint32_t m = (t & 1) ? mf : mr;
+            const bool two = pos[t] + 1u < end[t];
+            const uint32_t a = nib_of(w.nb, guard_id(c0[t], g.V, ex.ctl));
+            const uint32_t b = two ? nib_of(w.nb, guard_id(c1[t], g.V, ex.ctl)) : 0u;
+            if constexpr (Ex::instr) scanned += two ? 2u : 1u;
+            if ((a & m) == want[t] || (two && (b & m) == want[t])) {
+                found |= 1u << t;
+                on &= ~(1u << t);
+            } else {
+                pos[t] += 2u;
+                if (pos[t] >= lim[t]) on &= ~(1u << t);
+            }
+        }
+    }
+    // the rest of long lists by the whole warp, one search at a time
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        unsigned hm = __ballot_sync(FULL, ((any & ~found) >> t & 1u) && end[t] > pos[t]);
+        const uint32_t *C = (t & 1) ? g.Fc : g.Bc;
+        const uint32_t m = (t & 1) ? mf : mr;
+        while (hm) {
+            const unsigned j = __ffs(hm) - 1u;
+            hm &= hm - 1u;
+            const uint32_t bj = __shfl_sync(FULL, pos[t], j), ej = __shfl_sync(FULL, end[t], j);
+            const uint32_t wj = __shfl_sync(FULL, want[t], j);
+            for (uint32_t b = bj; b < ej; b += 32u) {
+                const uint32_t e = b + lane_id();
+                const bool hit = e < ej && (nib_of(w.nb, guard_id(__ldg(&C[e]), g.V, ex.ctl)) & m) == wj;
+                if constexpr (Ex::instr) scanned += lane_id() == 0 ? min(32u, ej - b) : 0u;
+                if (__ballot_sync(FULL, hit)) {
+                    if (lane_id() == j) found |= 1u << t;
+                    break;
+                }
+            }
+        }
+    }
+    if constexpr (Ex::instr) count_edges(ex, __reduce_add_sync(FULL, scanned));
     return found;
 }
 
-// Up to two live same-range neighbours of x in (R, C); *first gets the
-// first one (scc_kernels.cu:250-261).
-__device__ __forceinline__ uint32_t count_upto2(const uint32_t *st, const uint32_t *__restrict__ R,
+// ---------------------------------------------------------------------
+// init: every vertex live (the reference's cudaMemset of range and tags,
+// scc_WCC.cu:630-631), or, with trim, every vertex that has an in- and an
+// out-arc: with every vertex live the first trim-1 sweep is decided by the
+// degrees alone (scc_kernels.cu:187-233).  Eight ids per lane, one nibble
+// word: 128-bit offset loads, half a byte written per vertex.  Also checks
+// the offsets (the reference layout: Fr[0] = Fr[1] = 0, non-decreasing,
+// Fr[V+1] = E, load.cpp:55-77; same for Br) and sets the error before the
+// barrier, so no later pass runs on a bad graph; counts the live vertices
+// (C_LIST) and folds the first pivot's key over them.  What bounds it is
+// reading the offsets; a trimmed vertex's label is its own id and is not
+// written here (nibble 0).  R-MAT scale 22: with a state word, a label and a
+// live list written per vertex 21.8 us, now 12.4 us (33.5 MB of offsets).
+// ---------------------------------------------------------------------
+template <class Ex>
+__device__ bool ph_init(Ex &ex, const Graph &g, const Work &w, bool trim, bool stamps)
+{
+    return run_pass(ex, PH_INIT, [&](unsigned, unsigned nxt) {
+        if (ex.leader() && (g.Fr[0] != 0u || g.Fr[1] != 0u || g.Br[0] != 0u || g.Br[1] != 0u ||
+                            g.Fr[g.V + 1] != g.E || g.Br[g.V + 1] != g.E))
+            set_error(ex.ctl, E_BAD_GRAPH, 62);
+        unsigned long long best = 0;
+        uint32_t dmax = 0, nlive = 0, ntrim = 0, nv = 0;
+        bool bad = false;
+        const uint32_t nwords = (g.V / 32u + 1u) * 4u;   // whole units
+        for (uint32_t wd = ex.tid(); wd < nwords; wd += ex.nthr()) {
+            const uint32_t i0 = wd * 8u;
+            uint32_t x = 0;
+            if (i0 > g.V) {
+                w.nb[wd] = 0u;
+                continue;
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < 2u; q++) {
+                uint32_t f[5], b[5];
+                load_off5(g.Fr, i0 + 4u * q, g.V, g.vec, f);
+                load_off5(g.Br, i0 + 4u * q, g.V, g.vec, b);
+#pragma unroll
+                for (uint32_t j = 0; j < 4u; j++) {
+                    const uint32_t v = i0 + 4u * q + j;
+                    if (v < 1u || v > g.V) continue;
+                    bad |= f[j] > f[j + 1] || b[j] > b[j + 1];
+                    const uint32_t out = f[j + 1] - f[j], in = b[j + 1] - b[j];
+                    dmax = max(dmax, max(out, in));
+                    if (trim && (out == 0u || in == 0u)) {
+                        ntrim++;
+                        continue;
+                    }
+                    nlive++;
+                    x |= NL << (16u * q + 4u * j);
+                    const unsigned long long k = ((unsigned long long)(out * in) << 32) | (0xFFFFFFFFu - v);
+                    best = k > best ? k : best;
+                }
+            }
+            w.nb[wd] = x;
+            if (stamps && x) {   // trim-1 work lists stamp the live vertices
+                if (i0 + 7u <= g.V) {
+                    *reinterpret_cast<uint4 *>(w.st + i0) = make_uint4(0u, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4 *>(w.st + i0 + 4u) = make_uint4(0u, 0u, 0u, 0u);
+                } else {
+                    for (uint32_t i = i0; i <= g.V; i++) w.st[i] = 0u;
+                }
+            }
+            nv += min(8u, g.V + 1u - i0);
+        }
+        if (bad) set_error(ex.ctl, E_BAD_GRAPH, 61);
+        count_verts_n(ex, nv);
+        bq_add_edges(0, nlive);
+        bq_add_edges(1, ntrim);
+        block_max_atomic(best, &w.pivkey[0], dmax, Ex::grid ? &ex.ctl->maxdeg : nullptr);
+        if (threadIdx.x == 0) {
+            if (sccb_dsmem[12]) atomicAdd(&ex.lc(nxt)[C_LIST], sccb_dsmem[12]);
+            if (sccb_dsmem[13]) atomicAdd(&ex.ctl->n_trim1, (unsigned long long)sccb_dsmem[13]);
+            sccb_dsmem[12] = sccb_dsmem[13] = 0u;
+        }
+    });
+}
+
+// ---------------------------------------------------------------------
+// trim1 iterated to its fixpoint (vHong / wHong, scc_WCC.cu:680-687,
+// :773-780, :808-815).  Pass 0 checks every live vertex (all: by id, off the
+// nibble units, n of them) or a list; a trimmed vertex queues its live neighbours of the
+// same class for the next pass (stamped with the pass, so none is listed
+// twice; a vertex that is being checked meanwhile is listed all the same),
+// so later passes only recheck vertices that lost a neighbour.  A vertex is checked by searching both its lists for one live
+// neighbour, as in a bottom-up step: the first entries usually hold one.
+// Checking the live vertices instead of walking the lists of the vertices
+// that the degrees trim, R-MAT scale 20 with permuted ids (602,000 of
+// 1,048,576 trimmed): 58 us for the first pass,
+// now 21 us.
+// ---------------------------------------------------------------------
+template <class Ex>
+__device__ __forceinline__ void trim1_check(Ex &ex, const Graph &g, const Work &w, const bool (&in)[2],
+                                            const uint32_t (&v)[2], unsigned par, unsigned nxt)
+{
+    uint32_t s[2], pos[4], end[4], want[4];
+    bool ok[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) s[h] = in[h] ? nib_of(w.nb, v[h]) : 0u;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        ok[h] = (s[h] & NL) != 0u;
+        pos[2 * h] = ok[h] ? __ldg(&g.Br[v[h]]) : 0u;
+        end[2 * h] = ok[h] ? __ldg(&g.Br[v[h] + 1u]) : 0u;
+        pos[2 * h + 1] = ok[h] ? __ldg(&g.Fr[v[h]]) : 0u;
+        end[2 * h + 1] = ok[h] ? __ldg(&g.Fr[v[h] + 1u]) : 0u;
+        want[2 * h] = want[2 * h + 1] = s[h] & NCLASS;
+        count_verts(ex, in[h]);
+    }
+    const uint32_t found = find4(ex, g, w, pos, end, NCLASS, NCLASS, want);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const bool trim = ok[h] && (found >> (2 * h) & 3u) != 3u;
+        const unsigned m = __ballot_sync(FULL, trim);
+        if (m == 0u) continue;
+        if (trim) {
+            nib_kill(w.nb, v[h]);
+            w.label[v[h]] = v[h] | LBL_SELF;
+        }
+        if (lane_id() == 0) atomicAdd(&ex.ctl->n_trim1, (unsigned long long)__popc(m));
+        const uint32_t r = s[h] & NCLASS, tag = ex.gl + 1u;
+        // its live neighbours lost an in- or out-neighbour: the warp walks
+        // all the lists together, 64 entries per step
+        auto fn2 = [&](bool v0, uint32_t u0, uint32_t r0, bool v1, uint32_t u1, uint32_t r1) {
+            if (v0) u0 = guard_id(u0, g.V, ex.ctl);
+            if (v1) u1 = guard_id(u1, g.V, ex.ctl);
+            const bool p0 = v0 && (nib_of(w.nb, u0) & NCLASS) == r0 && stamp_claim(w.st, u0, tag);
+            const bool p1 = v1 && (nib_of(w.nb, u1) & NCLASS) == r1 && stamp_claim(w.st, u1, tag);
+            bq_push(0, p0, u0, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 11);
+            bq_push(0, p1, u1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 11);
+        };
+#pragma unroll
+        for (int dir = 0; dir < 2; dir++) {
+            const uint32_t *R = dir ? g.Br : g.Fr;
+            const uint32_t *C = dir ? g.Bc : g.Fc;
+            const uint32_t beg = trim ? __ldg(&R[v[h]]) : 0u;
+            const uint32_t deg = trim ? __ldg(&R[v[h] + 1]) - beg : 0u;
+            count_edges(ex, lbs_expand2(beg, deg, r, C, fn2));
+        }
+    }
+}
+
+template <class Ex>
+__device__ bool ph_trim1_fix(Ex &ex, const Graph &g, const Work &w, VList src0, bool all)
+{
+    uint32_t nq = src0.n;
+    for (unsigned it = 0;; it++) {
+        if (it > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 30); return false; }
+        const bool ok = run_pass(ex, PH_TRIM1_FIX, [&](unsigned, unsigned nxt) {
+            const unsigned par = ex.gl & 1u;
+            if (all && it == 0u) {
+                const uint32_t nu = g.V / 32u + 1u, cu = unit_group(ex, g.V, src0.n), ni = (nu + cu - 1u) / cu;
+                for (uint32_t i = ex.wid(); i < ni; i += ex.nwarps()) {
+                    const uint32_t u = lane_id() * ni + i;
+                    unit_walk2(u, load_unit(w, lane_id() < cu && u < nu, u).live,
+                               [&](const bool (&in)[2], const uint32_t (&v)[2], const unsigned (&)[2]) {
+                                   trim1_check(ex, g, w, in, v, par, nxt);
+                               });
+                }
+            } else {
+                const uint32_t *src = it == 0u ? src0.p : w.Q[0][par ^ 1u];
+                const uint32_t gs = item_group(ex, (nq + 1u) / 2u);
+                for (uint32_t base = ex.wid() * 2u * gs; base < nq; base += ex.nwarps() * 2u * gs) {
+                    bool in[2];
+                    uint32_t v[2];
+#pragma unroll
+                    for (uint32_t h = 0; h < 2u; h++) {
+                        const uint32_t i = base + h * gs + lane_id();
+                        in[h] = lane_id() < gs && i < nq;
+                        v[h] = in[h] ? src[i] : 0u;
+                    }
+                    trim1_check(ex, g, w, in, v, par, nxt);
+                }
+            }
+            bq_flush(1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], nullptr, nullptr, g.V, ex.ctl);
+        });
+        if (!ok) return false;
+        nq = last_count(ex, C_FQ);
+        if (nq == 0u) return true;
+    }
+}
+
+// Up to two live neighbours of x in class r in (R, C); *first gets the first
+// one (scc_kernels.cu:250-261).
+__device__ __forceinline__ uint32_t count_upto2(const uint32_t *nb, const uint32_t *__restrict__ R,
                                                 const uint32_t *__restrict__ C, uint32_t x,
                                                 uint32_t r, uint32_t *first, uint32_t V, Ctl *ctl)
 {
     uint32_t n = 0;
     for (uint32_t e = __ldg(&R[x]), end = __ldg(&R[x + 1]); e < end; e++) {
         uint32_t u = guard_id(__ldg(&C[e]), V, ctl);
-        if ((st[u] & RMASK) == r) {
+        if ((nib_of(nb, u) & NCLASS) == r) {
             n++;
             if (n == 2u) break;
             if (first) *first = u;
@@ -94,224 +443,27 @@ __device__ __forceinline__ uint32_t count_upto2(const uint32_t *st, const uint32
 
 // trim2 decision for v (scc_kernels.cu:236-348): the partner k, possibly v
 // itself through a self-loop, or 0.
-__device__ __forceinline__ uint32_t trim2_partner(const Graph &g, const uint32_t *st, uint32_t v, uint32_t r, Ctl *c)
+__device__ __forceinline__ uint32_t trim2_partner(const Graph &g, const uint32_t *nb, uint32_t v, uint32_t r, Ctl *c)
 {
     uint32_t k = 0;
-    if (count_upto2(st, g.Br, g.Bc, v, r, &k, g.V, c) == 1u) {
+    if (count_upto2(nb, g.Br, g.Bc, v, r, &k, g.V, c) == 1u) {
         for (uint32_t e = __ldg(&g.Fr[v]), end = __ldg(&g.Fr[v + 1]); e < end; e++) {
             if (__ldg(&g.Fc[e]) == k) {
-                if (count_upto2(st, g.Br, g.Bc, k, r, nullptr, g.V, c) == 1u) return k;
+                if (count_upto2(nb, g.Br, g.Bc, k, r, nullptr, g.V, c) == 1u) return k;
                 break;
             }
         }
     }
     k = 0;
-    if (count_upto2(st, g.Fr, g.Fc, v, r, &k, g.V, c) == 1u) {
+    if (count_upto2(nb, g.Fr, g.Fc, v, r, &k, g.V, c) == 1u) {
         for (uint32_t e = __ldg(&g.Br[v]), end = __ldg(&g.Br[v + 1]); e < end; e++) {
             if (__ldg(&g.Bc[e]) == k) {
-                if (count_upto2(st, g.Fr, g.Fc, k, r, nullptr, g.V, c) == 1u) return k;
+                if (count_upto2(nb, g.Fr, g.Fc, k, r, nullptr, g.V, c) == 1u) return k;
                 break;
             }
         }
     }
     return 0;
-}
-
-// ---------------------------------------------------------------------
-// init: every vertex live in range 0 (the reference's cudaMemset of range
-// and tags, scc_WCC.cu:630-631); optionally fold the first-pivot key.
-// ---------------------------------------------------------------------
-template <class Ex>
-__device__ bool ph_init(Ex &ex, const Graph &g, const Work &w, bool fold_pivot)
-{
-    // Also checks the offsets (the reference layout: Fr[0] = Fr[1] = 0,
-    // non-decreasing, Fr[V+1] = E, load.cpp:55-77; same for Br).  A bad
-    // graph sets the error before the barrier, so no later pass runs.
-    // Four ids per lane: 128-bit offset loads and state stores.
-    return run_pass(ex, PH_INIT, [&](unsigned, unsigned) {
-        unsigned long long best = 0;
-        if (ex.leader() && (g.Fr[0] != 0u || g.Fr[1] != 0u || g.Br[0] != 0u || g.Br[1] != 0u ||
-                            g.Fr[g.V + 1] != g.E || g.Br[g.V + 1] != g.E))
-            set_error(ex.ctl, E_BAD_GRAPH, 62);
-        bool bad = false;
-        uint32_t dmax = 0;
-        for (uint32_t i0 = ex.tid() * 4u; i0 <= g.V; i0 += ex.nthr() * 4u) {
-            uint32_t f[5], b[5];
-            load_off5(g.Fr, i0, g.V, g.vec, f);
-            load_off5(g.Br, i0, g.V, g.vec, b);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint32_t i = i0 + (uint32_t)j;
-                if (i <= g.V) {
-                    bad |= f[j] > f[j + 1] || b[j] > b[j + 1];
-                    dmax = max(dmax, max(f[j + 1] - f[j], b[j + 1] - b[j]));
-                    if (fold_pivot && i != 0u) {
-                        unsigned long long k = ((unsigned long long)((f[j + 1] - f[j]) * (b[j + 1] - b[j])) << 32) |
-                                               (0xFFFFFFFFu - i);
-                        best = k > best ? k : best;
-                    }
-                }
-            }
-            if (i0 + 3u <= g.V) {
-                *reinterpret_cast<uint4 *>(w.st + i0) = make_uint4(i0 == 0u ? DEAD : 0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4 *>(w.stamp + i0) = make_uint4(0u, 0u, 0u, 0u);
-            } else {
-                for (uint32_t i = i0; i <= g.V; i++) {
-                    w.st[i] = (i == 0u) ? DEAD : 0u;
-                    w.stamp[i] = 0u;
-                }
-            }
-        }
-        if (bad) set_error(ex.ctl, E_BAD_GRAPH, 61);
-        if (fold_pivot) block_max_atomic(best, &w.pivkey[0], dmax, Ex::nbq > 2 ? &ex.ctl->maxdeg : nullptr);
-        else if constexpr (Ex::nbq > 2) block_max_atomic32(dmax, &ex.ctl->maxdeg);
-    });
-}
-
-// ---------------------------------------------------------------------
-// init and trim1-once in one sweep (vSlota / wSlota with trim1): with every
-// vertex live in range 0, trim1 is decided by the degrees alone, so the
-// offsets the init pass validates also decide each vertex's first state.
-// Four ids per lane: 128-bit offset loads and 128-bit stores of st and
-// label (a trimmed vertex is labelled with itself, LBL_SELF).  Stamps are
-// cleared later for the few vertices that need them (ph_slota_first_update)
-// and smin entries when their representative is seeded, so this sweep
-// writes two vertex arrays, not four.  Survivors are compacted into Lout and
-// bid for the first pivot.  A bad graph sets the error before the barrier,
-// as in ph_init.
-// ---------------------------------------------------------------------
-template <class Ex>
-__device__ bool ph_init_trim1(Ex &ex, const Graph &g, const Work &w, uint32_t *Lout)
-{
-    return run_pass(ex, PH_TRIM1_ONCE, [&](unsigned, unsigned nxt) {
-        if (ex.leader() && (g.Fr[0] != 0u || g.Fr[1] != 0u || g.Br[0] != 0u || g.Br[1] != 0u ||
-                            g.Fr[g.V + 1] != g.E || g.Br[g.V + 1] != g.E))
-            set_error(ex.ctl, E_BAD_GRAPH, 62);
-        unsigned long long best = 0;
-        unsigned ntrim = 0;
-        bool bad = false;
-        uint32_t dmax = 0;
-        for (uint32_t base = ex.wid() * 128u; base <= g.V; base += ex.nwarps() * 128u) {
-            const uint32_t i0 = base + 4u * lane_id();
-            uint32_t f[5], b[5];
-            if (i0 <= g.V) {
-                load_off5(g.Fr, i0, g.V, g.vec, f);
-                load_off5(g.Br, i0, g.V, g.vec, b);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 5; j++) f[j] = b[j] = 0u;
-            }
-            uint32_t st4[4], lb4[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint32_t v = i0 + (uint32_t)j;
-                const bool valid = v >= 1u && v <= g.V;
-                bool surv = false;
-                st4[j] = DEAD;
-                lb4[j] = v;
-                if (v <= g.V) bad |= f[j] > f[j + 1] || b[j] > b[j + 1];
-                if (valid) {
-                    const uint32_t indeg = b[j + 1] - b[j], outdeg = f[j + 1] - f[j];
-                    dmax = max(dmax, max(indeg, outdeg));
-                    if (indeg == 0u || outdeg == 0u) {
-                        lb4[j] = v | LBL_SELF;   // a trimmed vertex is its own SCC
-                        ntrim++;
-                    } else {
-                        surv = true;
-                        st4[j] = 0u;
-                        unsigned long long k = ((unsigned long long)(outdeg * indeg) << 32) | (0xFFFFFFFFu - v);
-                        best = k > best ? k : best;
-                    }
-                }
-                bq_push(0, surv, v, w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 10);
-            }
-            if (i0 + 3u <= g.V) {
-                *reinterpret_cast<uint4 *>(w.st + i0) = make_uint4(st4[0], st4[1], st4[2], st4[3]);
-                *reinterpret_cast<uint4 *>(w.label + i0) = make_uint4(lb4[0], lb4[1], lb4[2], lb4[3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const uint32_t i = i0 + (uint32_t)j;
-                    if (i <= g.V) {
-                        w.st[i] = st4[j];
-                        w.label[i] = lb4[j];
-                    }
-                }
-            }
-            count_verts_n(ex, i0 <= g.V ? min(4u, g.V + 1u - i0) : 0u);
-        }
-        if (bad) set_error(ex.ctl, E_BAD_GRAPH, 61);
-        ntrim = __reduce_add_sync(FULL, ntrim);
-        if (lane_id() == 0 && ntrim) atomicAdd(&ex.ctl->n_trim1, (unsigned long long)ntrim);
-        block_max_atomic(best, &w.pivkey[0], dmax, Ex::nbq > 2 ? &ex.ctl->maxdeg : nullptr);
-        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl);
-    });
-}
-
-// ---------------------------------------------------------------------
-// trim1 iterated to its fixpoint (vHong / wHong, scc_WCC.cu:680-687,
-// :773-780, :808-815).  Pass 0 checks src0; a trimmed vertex queues its
-// live same-range neighbours for the next pass (stamp-deduplicated), so
-// later passes only recheck vertices that lost a neighbour.
-// ---------------------------------------------------------------------
-template <class Ex>
-__device__ bool ph_trim1_fix(Ex &ex, const Graph &g, const Work &w, VList src0, bool all_live)
-{
-    uint32_t nq = 0;
-    bool first = true;
-    for (unsigned it = 0;; it++) {
-        if (it > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 30); return false; }
-        bool ok = run_pass(ex, PH_TRIM1_FIX, [&](unsigned, unsigned nxt) {
-            const unsigned par = ex.gl & 1u;
-            const uint32_t tag = ex.gl + 1u;
-            VList src = first ? src0 : VList{w.Q[0][par ^ 1u], nq, 0u};
-            for (uint32_t base = ex.wid() * 32u; base < src.n; base += ex.nwarps() * 32u) {
-                uint32_t i = base + lane_id();
-                bool valid = i < src.n, trim = false;
-                uint32_t v = valid ? src.at(i) : 0u, r = 0u;
-                if (valid) {
-                    uint32_t s = w.st[v];
-                    if (s != DEAD) {
-                        r = s & RMASK;
-                        if (first && all_live)   // every vertex live in range 0: degrees decide
-                            trim = __ldg(&g.Br[v + 1]) == __ldg(&g.Br[v]) || __ldg(&g.Fr[v + 1]) == __ldg(&g.Fr[v]);
-                        else
-                            trim = !has_live(ex, w.st, g.Br, g.Bc, v, r, g.V) ||
-                                   !has_live(ex, w.st, g.Fr, g.Fc, v, r, g.V);
-                        if (trim) { w.st[v] = DEAD; w.label[v] = v | LBL_SELF; }
-                    }
-                }
-                count_verts(ex, valid);
-                unsigned m = __ballot_sync(FULL, trim);
-                if (lane_id() == 0 && m) atomicAdd(&ex.ctl->n_trim1, (unsigned long long)__popc(m));
-                if (m == 0u) continue;
-                // queue the live same-range neighbours of the trimmed vertices
-                // (they lost an in- or out-neighbour): the warp walks all their
-                // lists together, 64 entries per step
-                auto fn2 = [&](bool v0, uint32_t u0, uint32_t r0, bool v1, uint32_t u1, uint32_t r1) {
-                    if (v0) u0 = guard_id(u0, g.V, ex.ctl);
-                    if (v1) u1 = guard_id(u1, g.V, ex.ctl);
-                    const bool p0 = v0 && (w.st[u0] & RMASK) == r0 && stamp_claim(w.stamp, u0, tag);
-                    const bool p1 = v1 && (w.st[u1] & RMASK) == r1 && stamp_claim(w.stamp, u1, tag);
-                    bq_push(0, p0, u0, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 11);
-                    bq_push(0, p1, u1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 11);
-                };
-#pragma unroll
-                for (int dir = 0; dir < 2; dir++) {
-                    const uint32_t *R = dir ? g.Br : g.Fr;
-                    const uint32_t *C = dir ? g.Bc : g.Fc;
-                    const uint32_t beg = trim ? __ldg(&R[v]) : 0u;
-                    const uint32_t deg = trim ? __ldg(&R[v + 1]) - beg : 0u;
-                    count_edges(ex, lbs_expand2(beg, deg, r, C, fn2));
-                }
-            }
-            bq_flush(1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], nullptr, nullptr, g.V, ex.ctl);
-        });
-        if (!ok) return false;
-        first = false;
-        nq = last_count(ex, C_FQ);
-        if (nq == 0u) return true;
-    }
 }
 
 // ---------------------------------------------------------------------
@@ -325,14 +477,15 @@ __device__ bool ph_trim2(Ex &ex, const Graph &g, const Work &w, VList src)
 {
     bool ok = run_pass(ex, PH_TRIM2, [&](unsigned, unsigned nxt) {
         const unsigned par = ex.gl & 1u;
-        for (uint32_t base = ex.wid() * 32u; base < src.n; base += ex.nwarps() * 32u) {
+        const uint32_t gs = item_group(ex, src.n);
+        for (uint32_t base = ex.wid() * gs; base < src.n; base += ex.nwarps() * gs) {
             uint32_t i = base + lane_id();
-            bool valid = i < src.n, hit = false, cnt = false;
+            bool valid = lane_id() < gs && i < src.n, hit = false, cnt = false;
             uint32_t v = valid ? src.at(i) : 0u;
             if (valid) {
-                uint32_t s = w.st[v];
-                if (s != DEAD) {
-                    uint32_t k = trim2_partner(g, w.st, v, s & RMASK, ex.ctl);
+                const uint32_t s = nib_of(w.nb, v);
+                if (s & NL) {
+                    uint32_t k = trim2_partner(g, w.nb, v, s & NCLASS, ex.ctl);
                     if (k) {
                         hit = true;
                         cnt = v <= k;
@@ -349,103 +502,113 @@ __device__ bool ph_trim2(Ex &ex, const Graph &g, const Work &w, VList src)
     });
     if (!ok) return false;
     const uint32_t nT = last_count(ex, C_LIST);
+    if (nT == 0u) return true;
     return run_pass(ex, PH_TRIM2_APPLY, [&](unsigned, unsigned) {
         const uint32_t *T = w.Q[0][(ex.gl & 1u) ^ 1u];
-        for (uint32_t i = ex.tid(); i < nT; i += ex.nthr()) w.st[T[i]] = DEAD;
+        for (uint32_t i = ex.tid(); i < nT; i += ex.nthr()) nib_kill(w.nb, T[i]);
     });
 }
 
 // ---------------------------------------------------------------------
-// Frontier expansion of one direction for the lanes of a warp.  A lane with
-// act holds vertex v of range r; its neighbours that are live, in range r
-// and not yet visited in this direction are claimed with atomicOr and
-// appended to the next frontier (warp ballot compaction).  Vertices with
-// more than HEAVY_T entries are cut into CH-entry chunks for the next pass.
-// This is fwd/bwd (scc_kernels.cu:360-445) and fwd_warp/bwd_warp
-// (include/scc_kernels.h:46-105) over a queue instead of a full sweep.
+// The first FW-BW search (fwd/bwd, scc_kernels.cu:360-445, and
+// fwd_warp/bwd_warp, include/scc_kernels.h:46-105) over queues instead of
+// full sweeps.  Every vertex is in one range, so an arc is decided by half a
+// byte of its neighbour: live, and not yet visited in this direction; it is
+// claimed with atomicOr and appended to the next frontier (warp ballot
+// compaction).  At eight vertices a word the states of 16.8M vertices take
+// 8.4 MB and stay in L2 (a 32-bit word each: 67 MB, most gathers a DRAM
+// sector).  Vertices with more than HEAVY_T entries are cut into CH-entry
+// chunks for the next pass.
+//
+// K arcs per lane: all gathers, then all claims are issued before any
+// append.  eager (a short frontier, where a level's time is its chain of
+// dependent accesses): the claim is made without looking first -- a visited
+// bit on a vertex that is not live means nothing -- and the offsets of the
+// vertex are brought into L1 beside it, for the warp that goes on with it.  cnt (uniform over the CTA) adds the claimed vertices' degrees to
+// the pass's frontier-edge tally; a pass whose claims cannot reach the
+// bottom-up threshold skips those offset gathers.
 // ---------------------------------------------------------------------
-template <class Ex>
-__device__ __forceinline__ void bfs_edge_visit(Ex &ex, const Graph &g, const Work &w, int dir, bool valid,
-                                               uint32_t nbr, uint32_t r, unsigned par, unsigned nxt, bool cnt)
+template <int K, class Ex>
+__device__ __forceinline__ void bfs_visit(Ex &ex, const Graph &g, const Work &w, int dir, const bool (&v)[K],
+                                          uint32_t (&n)[K], unsigned par, unsigned nxt, bool cnt, bool eager = false)
 {
-    const uint32_t bit = dir ? BVB : FVB;
-    bool claim = false;
-    uint32_t done = 0xFFFFFFFFu;
-    if (valid) {
-        nbr = guard_id(nbr, g.V, ex.ctl);
-        uint32_t s = w.st[nbr];
-        if ((s & (RMASK | bit)) == r) {
-            const uint32_t o = atomicOr(&w.st[nbr], bit);
-            claim = !(o & bit);
-            done = completed(o, bit, nbr);
-        }
-    }
-    fold_completed(done);
+    const uint32_t bit = dir ? NB : NF;
     const uint32_t *Rn = dir ? g.Br : g.Fr;
-    if (cnt) bq_add_edges((unsigned)dir, claim ? __ldg(&Rn[nbr + 1]) - __ldg(&Rn[nbr]) : 0u);
-    bq_push((unsigned)dir, claim, nbr, w.qcap, w.Q[dir][par], &ex.lc(nxt)[C_FQ + dir], g.V, ex.ctl, 13);
-}
-
-// Two adjacency entries per lane: both gathers and both claims are issued
-// before either append, so every lane keeps two requests in flight.  cnt
-// (uniform over the CTA) adds the claimed vertices' degrees to the pass's
-// frontier-edge tally; a pass whose claims cannot reach the bottom-up
-// threshold skips those offset gathers.
-template <class Ex>
-__device__ __forceinline__ void bfs_edge_visit2(Ex &ex, const Graph &g, const Work &w, int dir, bool v0, uint32_t n0,
-                                                uint32_t r0, bool v1, uint32_t n1, uint32_t r1, unsigned par,
-                                                unsigned nxt, bool cnt)
-{
-    const uint32_t bit = dir ? BVB : FVB;
-    if (v0) n0 = guard_id(n0, g.V, ex.ctl);
-    if (v1) n1 = guard_id(n1, g.V, ex.ctl);
-    const uint32_t s0 = v0 ? w.st[n0] : DEAD;
-    const uint32_t s1 = v1 ? w.st[n1] : DEAD;
-    const bool t0 = v0 && (s0 & (RMASK | bit)) == r0;
-    const bool t1 = v1 && (s1 & (RMASK | bit)) == r1;
-    const uint32_t o0 = t0 ? atomicOr(&w.st[n0], bit) : bit;
-    const uint32_t o1 = t1 ? atomicOr(&w.st[n1], bit) : bit;
-    const bool c0 = !(o0 & bit), c1 = !(o1 & bit);
-    fold_completed(min(c0 ? completed(o0, bit, n0) : 0xFFFFFFFFu, c1 ? completed(o1, bit, n1) : 0xFFFFFFFFu));
-    // edges the claimed vertices will expand next (direction-switch rule)
-    if (cnt) {
-        const uint32_t *Rn = dir ? g.Br : g.Fr;
+    uint32_t x[K];
+    bool c[K];
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        if (v[j]) n[j] = guard_id(n[j], g.V, ex.ctl);
+        x[j] = !v[j] ? 0u : eager ? NL : nib_of(w.nb, n[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const bool t = (x[j] & (bit | NL)) == NL;
+        x[j] = t ? nib_or(w.nb, n[j], bit) : bit;
+        if (t && eager) prime_l1(Rn + n[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++) c[j] = (x[j] & (bit | NL)) == NL;
+    if (cnt) {   // edges the claimed vertices will expand next (direction-switch rule)
         unsigned e = 0;
-        if (c0) e += __ldg(&Rn[n0 + 1]) - __ldg(&Rn[n0]);
-        if (c1) e += __ldg(&Rn[n1 + 1]) - __ldg(&Rn[n1]);
+#pragma unroll
+        for (int j = 0; j < K; j++)
+            if (c[j]) e += __ldg(&Rn[n[j] + 1]) - __ldg(&Rn[n[j]]);
         bq_add_edges((unsigned)dir, e);
     }
-    bq_push((unsigned)dir, c0, n0, w.qcap, w.Q[dir][par], &ex.lc(nxt)[C_FQ + dir], g.V, ex.ctl, 13);
-    bq_push((unsigned)dir, c1, n1, w.qcap, w.Q[dir][par], &ex.lc(nxt)[C_FQ + dir], g.V, ex.ctl, 13);
+    bq_pushK<K>((unsigned)dir, c, n, w.qcap, w.Q[dir][par], &ex.lc(nxt)[C_FQ + dir], g.V, ex.ctl, 13);
 }
 
 template <class Ex>
-__device__ __forceinline__ void bfs_expand_lanes(Ex &ex, const Graph &g, const Work &w, int dir, uint32_t v,
-                                                 bool act, uint32_t r, int lw, unsigned par, unsigned nxt,
-                                                 bool cnt = true)
+__device__ __forceinline__ void bfs_visit2(Ex &ex, const Graph &g, const Work &w, int dir, bool v0, uint32_t n0,
+                                           bool v1, uint32_t n1, unsigned par, unsigned nxt, bool cnt)
+{
+    const bool v[2] = {v0, v1};
+    uint32_t n[2] = {n0, n1};
+    bfs_visit<2>(ex, g, w, dir, v, n, par, nxt, cnt);
+}
+
+// Frontier vertices, one per lane.  Lists of at most LANE_DEG entries are
+// walked by their own lanes, four entries a step (a low-degree frontier is
+// done in one or two rounds of gathers and needs no owner search); a warp
+// that holds a longer list, or at most 128 entries in all, walks the
+// concatenation of its lists, 128 entries a step.
+constexpr uint32_t LANE_DEG = 8;
+template <class Ex>
+__device__ __forceinline__ uint32_t bfs_expand_lanes(Ex &ex, const Graph &g, const Work &w, int dir, bool act,
+                                                     uint32_t v, unsigned par, unsigned nxt, bool cnt, bool eager,
+                                                     bool local = false)
 {
     const uint32_t *R = dir ? g.Br : g.Fr;
     const uint32_t *C = dir ? g.Bc : g.Fc;
-    uint32_t beg = 0, deg = 0;
-    if (act) { beg = __ldg(&R[v]); deg = __ldg(&R[v + 1]) - beg; }
-    bool heavy = deg > HEAVY_T;
-    uint32_t nch = heavy ? (deg + CH - 1u) / CH : 0u;
-    if (lw > 0 && (lane_id() & ((1u << lw) - 1u)) != 0u) nch = 0u;
-    warp_push_chunks(v, nch, w.H[dir][par], &ex.lc(nxt)[C_FH + dir], w.hcap, ex.ctl);
-    if (heavy) deg = 0u;
-    unsigned tot;
-    if (lw < 0) {
-        auto fn2 = [&](bool v0, uint32_t n0, uint32_t r0, bool v1, uint32_t n1, uint32_t r1) {
-            bfs_edge_visit2(ex, g, w, dir, v0, n0, r0, v1, n1, r1, par, nxt, cnt);
-        };
-        tot = lbs_expand2(beg, deg, r, C, fn2);
-    } else {
-        auto fn = [&](bool valid, uint32_t nbr, uint32_t rr) {
-            bfs_edge_visit(ex, g, w, dir, valid, nbr, rr, par, nxt, cnt);
-        };
-        tot = vw_expand(beg, deg, r, (unsigned)lw, C, fn);
+    const uint32_t beg = act ? __ldg(&R[v]) : 0u;
+    uint32_t deg = act ? __ldg(&R[v + 1u]) - beg : 0u;
+    count_verts(ex, act);
+    const uint32_t maxd = __reduce_max_sync(FULL, deg), total = __reduce_add_sync(FULL, deg);
+    if (cnt && local && lane_id() == 0) atomicSub(&sccb_dsmem[12 + dir], total);   // not in the next frontier any more
+    if (maxd <= LANE_DEG && (maxd <= 4u || total > 128u)) {
+        for (uint32_t k = 0; k < maxd; k += 4u) {
+            bool ok[4];
+            uint32_t n[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) {
+                ok[j] = k + j < deg;
+                n[j] = ok[j] ? __ldg(&C[beg + k + j]) : 0u;
+            }
+            bfs_visit<4>(ex, g, w, dir, ok, n, par, nxt, cnt, eager);
+        }
+        count_edges(ex, total);
+        return total;
     }
-    count_edges(ex, tot);
+    if (maxd > HEAVY_T) {
+        const bool heavy = deg > HEAVY_T;
+        warp_push_chunks(v, heavy ? (deg + CH - 1u) / CH : 0u, w.H[dir][par], &ex.lc(nxt)[C_FH + dir], w.hcap, ex.ctl);
+        if (heavy) deg = 0u;
+    }
+    count_edges(ex, lbs_walk4(beg, deg, C, [&](const bool (&ok)[4], uint32_t (&n)[4]) {
+        bfs_visit<4>(ex, g, w, dir, ok, n, par, nxt, cnt, eager);
+    }));
+    return total;
 }
 
 // Top-down expansion with the virtual-warp schedule (W = 1 << lw lanes per
@@ -454,9 +617,8 @@ __device__ __forceinline__ void bfs_expand_lanes(Ex &ex, const Graph &g, const W
 constexpr int VWK = 4;
 template <class Ex>
 __device__ __forceinline__ void bfs_expand_vwk(Ex &ex, const Graph &g, const Work &w, int dir,
-                                               const uint32_t (&v)[VWK], const bool (&act)[VWK],
-                                               const uint32_t (&r)[VWK], int lw, unsigned par, unsigned nxt,
-                                               bool cnt)
+                                               const uint32_t (&v)[VWK], const bool (&act)[VWK], int lw, unsigned par,
+                                               unsigned nxt, bool cnt)
 {
     const uint32_t *R = dir ? g.Br : g.Fr;
     const uint32_t *C = dir ? g.Bc : g.Fc;
@@ -474,16 +636,17 @@ __device__ __forceinline__ void bfs_expand_vwk(Ex &ex, const Graph &g, const Wor
                          &ex.lc(nxt)[C_FH + dir], w.hcap, ex.ctl);
         if (heavy) deg[j] = 0u;
     }
-    auto fn = [&](int j, bool v0, uint32_t n0, bool v1, uint32_t n1) {
-        bfs_edge_visit2(ex, g, w, dir, v0, n0, r[j], v1, n1, r[j + 1], par, nxt, cnt);
+    auto fn = [&](int, bool v0, uint32_t n0, bool v1, uint32_t n1) {
+        bfs_visit2(ex, g, w, dir, v0, n0, v1, n1, par, nxt, cnt);
     };
     count_edges(ex, vw_expandK<VWK>(beg, deg, (unsigned)lw, C, fn));
 }
 
-// One CH-entry chunk of a heavy vertex, expanded by the whole warp.
+// One CH-entry chunk of a heavy vertex, expanded by the whole warp:
+// fn(v0, n0, v1, n1).
 template <class Ex, class Fn>
 __device__ __forceinline__ void chunk_expand(Ex &ex, const uint32_t *__restrict__ R, const uint32_t *__restrict__ C,
-                                             uint2 hc, uint32_t aux, Fn &&fn)
+                                             uint2 hc, Fn &&fn)
 {
     uint32_t beg = __ldg(&R[hc.x]) + hc.y * CH;
     uint32_t end = min(__ldg(&R[hc.x + 1]), beg + CH);
@@ -492,163 +655,78 @@ __device__ __forceinline__ void chunk_expand(Ex &ex, const uint32_t *__restrict_
         const bool v0 = e0 < end, v1 = e1 < end;
         const uint32_t n0 = v0 ? __ldg(&C[e0]) : 0u;
         const uint32_t n1 = v1 ? __ldg(&C[e1]) : 0u;
-        fn(v0, n0, aux, v1, n1, aux);
+        fn(v0, n0, v1, n1);
     }
     count_edges(ex, end > beg ? end - beg : 0u);
 }
 
-// Bottom-up step over 64 vertices, both directions at once: entries
-// k*64 .. k*64+63 of `src` (the scope list, or the id range 1..V when the
-// scope holds most live vertices: coalesced state and offset loads, no list
-// indirection), two per lane.  Every lane keeps up to four searches in
-// flight (2 vertices x forward/backward), each testing two adjacency
-// entries per step, so a lane waits on one round of gathers for all of
-// them; a list longer than 32 entries gets its first 8 entries tested by
-// the lane (a visited neighbour is usually among the first, lowest ids) and
-// the rest by the whole warp.  A live vertex outside the scope can only
-// find a visited neighbour of its own range if its range is being
-// searched, so walking ids reaches the same set as walking the scope.
-//
-// With sout set (whole-GPU policy), every live vertex of the item that is
-// still unvisited in a direction of the search is appended to sout (staging
-// queue 2): the scope of the next bottom-up step, which then walks only
-// those instead of the whole scope.
+// Bottom-up step over the warp's units, both directions at once: every live
+// vertex still unvisited in a direction that goes bottom-up (puf forward,
+// pub backward) searches its lists for a visited neighbour.  The nibbles name
+// those vertices by themselves, so no scope list is kept or walked.  The live
+// vertices still unvisited in some direction are tallied (C_SCOPE): the scope
+// the next pass weighs its frontier against.
 template <class Ex>
-__device__ __forceinline__ void bfs_pull2(Ex &ex, const Graph &g, const Work &w, bool puf, bool pub, VList src,
-                                          uint32_t k, unsigned par, unsigned nxt, uint32_t *sout)
+__device__ __forceinline__ void bfs_pull(Ex &ex, const Graph &g, const Work &w, bool puf, bool pub, uint32_t u,
+                                         const NibUnit &x, unsigned par, unsigned nxt)
 {
-    constexpr uint32_t MF = RMASK | FVB, MB = RMASK | BVB;
-    uint32_t v[2], s[2], pos[4], end[4], want[4];
-    bool on[4], found[4], ok[2];
+    const uint32_t wf = puf ? x.live & ~x.fwd : 0u, wb = pub ? x.live & ~x.bwd : 0u;
+    uint32_t left = __popc(x.live & ~(x.fwd & x.bwd));
+    unit_walk2(u, wf | wb, [&](const bool (&in)[2], const uint32_t (&v)[2], const unsigned (&own)[2]) {
+        uint32_t pos[4], end[4];
+        const uint32_t want[4] = {NF, NB, NF, NB};
+        bool half[2];   // already visited the other way
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const uint32_t i = k * 64u + 32u * (uint32_t)h + lane_id();
-        ok[h] = i < src.n;
-        v[h] = ok[h] ? src.at(i) : 0u;
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) s[h] = ok[h] ? w.st[v[h]] : DEAD;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const bool live = s[h] != DEAD;
-        const bool nf = puf && live && !(s[h] & FVB);   // forward: a visited in-neighbour
-        const bool nb = pub && live && !(s[h] & BVB);   // backward: a visited out-neighbour
-        pos[2 * h] = nf ? __ldg(&g.Br[v[h]]) : 0u;
-        end[2 * h] = nf ? __ldg(&g.Br[v[h] + 1u]) : 0u;
-        pos[2 * h + 1] = nb ? __ldg(&g.Fr[v[h]]) : 0u;
-        end[2 * h + 1] = nb ? __ldg(&g.Fr[v[h] + 1u]) : 0u;
-        want[2 * h] = (s[h] & RMASK) | FVB;
-        want[2 * h + 1] = (s[h] & RMASK) | BVB;
-    }
-    unsigned scanned = 0;
-    uint32_t lim[4];   // the lane scans a list to its end if it is short, else its first entries
-    const uint32_t first = min(8u, w.pull_lane);
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-        found[t] = false;
-        on[t] = end[t] > pos[t];
-        lim[t] = end[t] - pos[t] <= w.pull_lane ? end[t] : pos[t] + first;
-    }
-    // by the lane: two entries of every open search per step (a visited
-    // neighbour is usually among the first entries, the lowest ids)
-    while (on[0] || on[1] || on[2] || on[3]) {
-        uint32_t c0[4], c1[4];
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            const uint32_t *C = (t & 1) ? g.Fc : g.Bc;
-            c0[t] = on[t] ? __ldg(&C[pos[t]]) : 0u;
-            c1[t] = on[t] && pos[t] + 1u < end[t] ? __ldg(&C[pos[t] + 1u]) : 0u;
+        for (int h = 0; h < 2; h++) {
+            const uint32_t b = v[h] & 31u;
+            const bool nf = in[h] & (__shfl_sync(FULL, wf, own[h]) >> b);   // forward: a visited in-neighbour
+            const bool nb = in[h] & (__shfl_sync(FULL, wb, own[h]) >> b);   // backward: a visited out-neighbour
+            half[h] = (__shfl_sync(FULL, x.fwd | x.bwd, own[h]) >> b) & 1u;
+            pos[2 * h] = nf ? __ldg(&g.Br[v[h]]) : 0u;
+            end[2 * h] = nf ? __ldg(&g.Br[v[h] + 1u]) : 0u;
+            pos[2 * h + 1] = nb ? __ldg(&g.Fr[v[h]]) : 0u;
+            end[2 * h + 1] = nb ? __ldg(&g.Fr[v[h] + 1u]) : 0u;
         }
+        const uint32_t found = find4(ex, g, w, pos, end, NF, NB, want);
 #pragma unroll
-        for (int t = 0; t < 4; t++) {
-            if (!on[t]) continue;
-            const uint32_t m = (t & 1) ? MB : MF;
-            const uint32_t a = w.st[guard_id(c0[t], g.V, ex.ctl)];
-            const uint32_t b = pos[t] + 1u < end[t] ? w.st[guard_id(c1[t], g.V, ex.ctl)] : DEAD;
-            if constexpr (Ex::instr) scanned += pos[t] + 1u < end[t] ? 2u : 1u;
-            if ((a & m) == want[t] || (b & m) == want[t]) {
-                found[t] = true;
-                on[t] = false;
-            } else {
-                pos[t] += 2u;
-                on[t] = pos[t] < lim[t];
+        for (int h = 0; h < 2; h++) {
+            const bool ff = found >> (2 * h) & 1u, fb = found >> (2 * h + 1) & 1u;
+            if (ff || fb) {
+                nib_or(w.nb, v[h], (ff ? NF : 0u) | (fb ? NB : 0u));
+                if ((ff && fb) || half[h]) left--;
             }
+            // frontier edges of the next level: out-degree forward, in-degree backward
+            if (puf) bq_add_edges(0u, ff ? __ldg(&g.Fr[v[h] + 1u]) - __ldg(&g.Fr[v[h]]) : 0u);
+            if (pub) bq_add_edges(1u, fb ? __ldg(&g.Br[v[h] + 1u]) - __ldg(&g.Br[v[h]]) : 0u);
+            count_verts(ex, in[h]);
+            if (puf) bq_push(0u, ff, v[h], w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 19);
+            if (pub) bq_push(1u, fb, v[h], w.qcap, w.Q[1][par], &ex.lc(nxt)[C_BQ], g.V, ex.ctl, 19);
         }
-    }
-    // the rest of long lists by the whole warp, one search at a time
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-        unsigned hm = __ballot_sync(FULL, !found[t] && end[t] > pos[t]);
-        const uint32_t *C = (t & 1) ? g.Fc : g.Bc;
-        const uint32_t m = (t & 1) ? MB : MF;
-        while (hm) {
-            const unsigned j = __ffs(hm) - 1u;
-            hm &= hm - 1u;
-            const uint32_t bj = __shfl_sync(FULL, pos[t], j), ej = __shfl_sync(FULL, end[t], j);
-            const uint32_t wj = __shfl_sync(FULL, want[t], j);
-            for (uint32_t b = bj; b < ej; b += 32u) {
-                const uint32_t e = b + lane_id();
-                const bool hit = e < ej && (w.st[guard_id(__ldg(&C[e]), g.V, ex.ctl)] & m) == wj;
-                if constexpr (Ex::instr) scanned += lane_id() == 0 ? min(32u, ej - b) : 0u;
-                if (__ballot_sync(FULL, hit)) {
-                    if (lane_id() == j) found[t] = true;
-                    break;
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const uint32_t bits = (found[2 * h] ? FVB : 0u) | (found[2 * h + 1] ? BVB : 0u);
-        fold_completed(bits ? completed(atomicOr(&w.st[v[h]], bits), bits, v[h]) : 0xFFFFFFFFu);
-        // frontier edges of the next level: out-degree forward, in-degree backward
-        if (puf) bq_add_edges(0u, found[2 * h] ? __ldg(&g.Fr[v[h] + 1u]) - __ldg(&g.Fr[v[h]]) : 0u);
-        if (pub) bq_add_edges(1u, found[2 * h + 1] ? __ldg(&g.Br[v[h] + 1u]) - __ldg(&g.Br[v[h]]) : 0u);
-        count_verts(ex, ok[h]);
-        if (puf) bq_push(0u, found[2 * h], v[h], w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 19);
-        if (pub) bq_push(1u, found[2 * h + 1], v[h], w.qcap, w.Q[1][par], &ex.lc(nxt)[C_BQ], g.V, ex.ctl, 19);
-        if (Ex::nbq > 2 && sout) {
-            const bool fv = (s[h] & FVB) || found[2 * h], bv = (s[h] & BVB) || found[2 * h + 1];
-            const bool keep = s[h] != DEAD && !(fv && bv);
-            bq_push(2u, keep, v[h], w.qcap, sout, &ex.lc(nxt)[C_SCOPE], g.V, ex.ctl, 25);
-        }
-    }
-    if constexpr (Ex::instr) {
-        unsigned t = __reduce_add_sync(FULL, scanned);
-        count_edges(ex, t);
-    }
+    });
+    bq_add_edges(2u, left);
 }
 
 // Forward and backward reachability from the first pivot p to closure.  Pass
 // 0 flags the pivot and expands it.  Each later pass picks, per direction,
-// top-down (expand the frontier queue and the heavy chunks) or bottom-up over
-// `scope` (the vertices the search can reach) when the frontier's vertices
-// have more than bu_k * scope.n edges to expand.  lw < 0 selects the
-// load-balanced warp schedule for top-down steps, lw >= 0 the virtual-warp
-// schedule with W = 1 << lw.
-//
-// On the whole-GPU policy every bottom-up step also lists the vertices of
-// its scope still unvisited in some direction (into w.S[0], w.S[1] in
-// turn): the next bottom-up step walks that shorter list, and the Beamer
-// rule weighs the frontier against it.  *last (optional) receives the scope
-// at the end: every live vertex of the original scope that is not visited
-// in both directions is in it.
+// top-down (expand the frontier queue and the heavy chunks) or bottom-up
+// (scan the unvisited live vertices) when the frontier's vertices have more
+// than bu_k * nscope edges to expand; nscope is the live count, and after
+// the first bottom-up step what that left unvisited.  lw < 0 selects the
+// warp schedule for top-down steps, lw >= 0 the virtual-warp schedule with
+// W = 1 << lw.
 template <class Ex>
-__device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw, VList scope, VList *last = nullptr)
+__device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw, uint32_t nscope)
 {
-    unsigned nshrink = 0;
-    const unsigned gsz = (lw < 0) ? 32u : (32u >> lw);
+    bool shrunk = false;
     bool ok = run_pass(ex, PH_BFS0, [&](unsigned, unsigned nxt) {
         const unsigned par = ex.gl & 1u;
         if (ex.leader()) {
-            if (completed(atomicOr(&w.st[p], FVB | BVB), FVB | BVB, p) == p) atomicMin(cta_first_min(), p);
+            nib_or(w.nb, p, NF | NB);
             atomicAdd(&ex.ctl->n_pivot, 1ull);
-            w.smin[p] = p;   // p represents its SCC: the update passes fold the members in
         }
         // the pivot is usually the largest hub: 64-entry pieces of its out-
         // and in-list, one per warp, so they spread over the whole grid in
         // one round of gathers
-        const uint32_t r = w.st[p] & RMASK;
         const uint32_t fb = __ldg(&g.Fr[p]), fe = __ldg(&g.Fr[p + 1]);
         const uint32_t bb = __ldg(&g.Br[p]), be = __ldg(&g.Br[p + 1]);
         const uint32_t nfc = (fe - fb + 63u) / 64u, nbc = (be - bb + 63u) / 64u;
@@ -658,9 +736,9 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
             const uint32_t end = min(beg + 64u, dir ? be : fe);
             const uint32_t *C = dir ? g.Bc : g.Fc;
             const uint32_t e0 = beg + lane_id(), e1 = e0 + 32u;
-            const bool v0 = e0 < end, v1 = e1 < end;
-            const uint32_t n0 = v0 ? __ldg(&C[e0]) : 0u, n1 = v1 ? __ldg(&C[e1]) : 0u;
-            bfs_edge_visit2(ex, g, w, dir, v0, n0, r, v1, n1, r, par, nxt, true);
+            // the pivot itself (a self-loop) is flagged by the leader alone
+            const uint32_t n0 = e0 < end ? __ldg(&C[e0]) : p, n1 = e1 < end ? __ldg(&C[e1]) : p;
+            bfs_visit2(ex, g, w, dir, n0 != p, n0, n1 != p, n1, par, nxt, true);
             count_edges(ex, end - beg);
         }
         bq_flush(2, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], w.Q[1][par], &ex.lc(nxt)[C_BQ], g.V, ex.ctl,
@@ -669,216 +747,145 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
     if (!ok) return false;
     // The claims of a pass are tallied by degree (the frontier edges Beamer's
     // rule weighs) only while they could reach the bottom-up threshold: a
-    // pass claims at most the edges it expands (and at most the scope), and
-    // each claim brings at most maxdeg edges.  Bit d of known: the previous
+    // pass is taken to leave at most four times the edges of its frontier (and
+    // at most the scope), and each claim brings at most maxdeg edges.  Bit d of known: the previous
     // pass tallied direction d, so its count is exact.  Whole-GPU policy
     // only: the single-CTA and batched searches are short, and there the
     // extra registers cost more than the gathers they save.
-    constexpr bool skip_tally = Ex::nbq > 2;
     unsigned known = 3u;
-    const uint32_t dmax32 = skip_tally ? __ldcg(&ex.ctl->maxdeg) : 0u;
+    const uint32_t dmax32 = Ex::grid ? __ldcg(&ex.ctl->maxdeg) : 0u;
     for (unsigned lev = 1;; lev++) {
         const uint32_t nf = last_count(ex, C_FQ), nb = last_count(ex, C_BQ);
         const uint32_t nhf = last_count(ex, C_FH), nhb = last_count(ex, C_BH);
-        if (nf + nb + nhf + nhb == 0u) {
-            if (last) *last = scope;
-            return true;
-        }
+        if (nf + nb + nhf + nhb == 0u) return true;
         if (lev > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 40); return false; }
         // Beamer's rule: bottom-up when the frontier has more edges to
         // expand than the scope has vertices to test (times bu_k)
         const uint32_t mf = last_count(ex, C_FE), mb = last_count(ex, C_BE);
-        const bool puf = w.bu_k && (unsigned long long)mf > (unsigned long long)scope.n * w.bu_k;
-        const bool pub = w.bu_k && (unsigned long long)mb > (unsigned long long)scope.n * w.bu_k;
+        const bool puf = w.bu_k && (unsigned long long)mf > (unsigned long long)nscope * w.bu_k;
+        const bool pub = w.bu_k && (unsigned long long)mb > (unsigned long long)nscope * w.bu_k;
         unsigned cm = 3u;   // bit d: this pass tallies direction d
-        if constexpr (skip_tally) {
+        if constexpr (Ex::grid) {
             cm = 0u;
             const unsigned long long dmax = dmax32;
 #pragma unroll
             for (int d = 0; d < 2; d++) {
                 const bool pu = d ? pub : puf;
                 const unsigned long long nfd = d ? nb : nf, mfd = d ? mb : mf, nhd = d ? nhb : nhf;
-                unsigned long long xe = pu ? scope.n : (((known >> d) & 1u) ? mfd : nfd * dmax) + nhd * CH;
-                xe = min(xe, (unsigned long long)scope.n);
-                if (w.bu_k && xe * dmax > (unsigned long long)scope.n * w.bu_k) cm |= 1u << d;
+                unsigned long long xe = pu ? nscope : 4u * ((((known >> d) & 1u) ? mfd : nfd * dmax) + nhd * CH);
+                xe = min(xe, (unsigned long long)nscope);
+                if (w.bu_k && xe * dmax > (unsigned long long)nscope * w.bu_k) cm |= 1u << d;
             }
             // a bottom-up step may shrink the scope the next pass weighs
             // against, so it tallies both directions (and its finds)
             if (puf || pub) cm = 3u;
             known = cm;
         }
-        // bottom-up steps (both directions in one sweep of 64-vertex items)
-        // walk the ids instead of the scope list when it holds most of them
-        const VList psrc = 2ull * scope.n >= (unsigned long long)g.V ? VList{nullptr, g.V, 1u} : scope;
-        const uint32_t nd = (puf || pub) ? (psrc.n + 63u) / 64u : 0u;
-        // one shrink per search: a second bottom-up step over the shrunken
-        // scope costs more than the top-down steps it would replace
-        uint32_t *sout = (Ex::nbq > 2 && (puf || pub) && nshrink == 0u) ? w.S[0] : nullptr;
         ok = run_pass(ex, (puf || pub) ? PH_BFS_PULL : PH_BFS, [&](unsigned, unsigned nxt) {
             const unsigned par = ex.gl & 1u, cp = par ^ 1u;
-            // virtual-warp items take VWK groups of frontier vertices
-            const uint32_t isz = (lw < 0) ? gsz : (uint32_t)VWK * gsz;
-            const uint32_t ngf = (nf + isz - 1u) / isz, ngb = (nb + isz - 1u) / isz;
+            if (puf || pub) {
+                // a warp's units lie far apart: where ids follow degree, the
+                // hubs' long lists spread over all warps (R-MAT scale 22, the
+                // first step: 256 adjacent vertices a warp 122 us, spread
+                // 86 us)
+                const uint32_t nu = g.V / 32u + 1u, cu = unit_group(ex, g.V, nscope), ni = (nu + cu - 1u) / cu;
+                for (uint32_t i = ex.wid(); i < ni; i += ex.nwarps()) {
+                    const uint32_t u = lane_id() * ni + i;
+                    bfs_pull(ex, g, w, puf, pub, u, load_unit(w, lane_id() < cu && u < nu, u), par, nxt);
+                }
+            }
+            // frontier vertices a warp takes at once: 1 << gsh (a virtual-warp
+            // item takes VWK = 4 groups of 32 >> lw)
+            const bool full = nf + nb >= 16u * ex.nwarps();   // work for every warp
+            const uint32_t gsh = lw >= 0 ? 7u - (uint32_t)lw : item_shift(ex, nf + nb);
+            const uint32_t ngf = (nf + (1u << gsh) - 1u) >> gsh, ngb = (nb + (1u << gsh) - 1u) >> gsh;
             const uint32_t items_f = puf ? 0u : nhf + ngf;
             const uint32_t items_b = pub ? 0u : nhb + ngb;
-            for (uint32_t it = ex.wid(); it < nd + items_f + items_b; it += ex.nwarps()) {
-                if (it < nd) {
-                    bfs_pull2(ex, g, w, puf, pub, psrc, it, par, nxt, sout);
-                    continue;
-                }
-                const uint32_t it2 = it - nd;
-                const int dir = it2 < items_f ? 0 : 1;
-                const uint32_t k = dir ? it2 - items_f : it2;
+            for (uint32_t it = ex.wid(); it < items_f + items_b; it += ex.nwarps()) {
+                const int dir = it < items_f ? 0 : 1;
+                const uint32_t k = dir ? it - items_f : it;
                 const uint32_t nh = dir ? nhb : nhf;
                 if (k < nh) {
-                    uint2 hc = w.H[dir][cp][k];
-                    uint32_t r = w.st[hc.x] & RMASK;
-                    auto fn2 = [&](bool v0, uint32_t n0, uint32_t r0, bool v1, uint32_t n1, uint32_t r1) {
-                        bfs_edge_visit2(ex, g, w, dir, v0, n0, r0, v1, n1, r1, par, nxt, (cm >> dir) & 1u);
+                    auto fn2 = [&](bool v0, uint32_t n0, bool v1, uint32_t n1) {
+                        bfs_visit2(ex, g, w, dir, v0, n0, v1, n1, par, nxt, (cm >> dir) & 1u);
                     };
-                    chunk_expand(ex, dir ? g.Br : g.Fr, dir ? g.Bc : g.Fc, hc, r, fn2);
+                    chunk_expand(ex, dir ? g.Br : g.Fr, dir ? g.Bc : g.Fc, w.H[dir][cp][k], fn2);
+                    continue;
+                }
+                const uint32_t n = dir ? nb : nf;
+                if (lw < 0) {
+                    const uint32_t i = ((k - nh) << gsh) + lane_id();
+                    const bool valid = lane_id() >> gsh == 0u && i < n;
+                    bfs_expand_lanes(ex, g, w, dir, valid, valid ? w.Q[dir][cp][i] : 0u, par, nxt, (cm >> dir) & 1u, !full);
                 } else {
-                    const uint32_t gi = k - nh;
-                    const uint32_t n = dir ? nb : nf;
-                    unsigned slot = (lw < 0) ? lane_id() : (lane_id() >> lw);
-                    uint32_t i = gi * isz + slot;
-                    bool valid = i < n;
-                    uint32_t v = valid ? w.Q[dir][cp][i] : 0u;
-                    uint32_t r = valid ? (w.st[v] & RMASK) : 0u;
-                    bool lead = (lw <= 0) || ((lane_id() & ((1u << lw) - 1u)) == 0u);
-                    if (lw < 0) {
-                        count_verts(ex, valid && lead);
-                        bfs_expand_lanes(ex, g, w, dir, v, valid, r, lw, par, nxt, (cm >> dir) & 1u);
-                    } else {
-                        uint32_t vk[VWK], rk[VWK];
-                        bool ak[VWK];
+                    const bool lead = (lane_id() & ((1u << lw) - 1u)) == 0u;
+                    uint32_t vk[VWK];
+                    bool ak[VWK];
 #pragma unroll
-                        for (int j = 0; j < VWK; j++) {
-                            const uint32_t ij = i + (uint32_t)j * gsz;
-                            ak[j] = ij < n;
-                            vk[j] = ak[j] ? w.Q[dir][cp][ij] : 0u;
-                        }
-#pragma unroll
-                        for (int j = 0; j < VWK; j++) {
-                            rk[j] = ak[j] ? (w.st[vk[j]] & RMASK) : 0u;
-                            count_verts(ex, ak[j] && lead);
-                        }
-                        bfs_expand_vwk(ex, g, w, dir, vk, ak, rk, lw, par, nxt, (cm >> dir) & 1u);
+                    for (int j = 0; j < VWK; j++) {
+                        const uint32_t ij = ((k - nh) << gsh) + (lane_id() >> lw) + (uint32_t)j * (32u >> lw);
+                        ak[j] = ij < n;
+                        vk[j] = ak[j] ? w.Q[dir][cp][ij] : 0u;
+                        count_verts(ex, ak[j] && lead);
+                    }
+                    bfs_expand_vwk(ex, g, w, dir, vk, ak, lw, par, nxt, (cm >> dir) & 1u);
+                }
+            }
+            if (lw < 0) {
+                for (int dir = 0; dir < 2; dir++) {
+                    if (dir ? pub : puf) continue;   // found bottom-up: left to the next pass
+                    uint32_t edges = 0;
+                    for (unsigned left = full ? FULL_ROUNDS : LOCAL_ROUNDS; left && edges < LOCAL_EDGES; left--) {
+                        uint32_t v;
+                        const unsigned took = bq_pop((unsigned)dir, w.qcap, full ? 24u : 1u, local_cap(w.qcap, full), v);
+                        if (took == 0u) break;
+                        edges += bfs_expand_lanes(ex, g, w, dir, lane_id() < took, v, par, nxt, (cm >> dir) & 1u, !full,
+                                                  true);
                     }
                 }
             }
-            bq_flush(sout ? 3u : 2u, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], w.Q[1][par],
-                     &ex.lc(nxt)[C_BQ], g.V, ex.ctl, &ex.lc(nxt)[C_FE], &ex.lc(nxt)[C_BE], sout,
-                     &ex.lc(nxt)[C_SCOPE]);
+            bq_flush(2, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], w.Q[1][par], &ex.lc(nxt)[C_BQ], g.V, ex.ctl,
+                     &ex.lc(nxt)[C_FE], &ex.lc(nxt)[C_BE], &ex.lc(nxt)[C_SCOPE]);
         });
         if (!ok) return false;
-        if (sout) {   // the next bottom-up steps walk the shrunken scope
-            scope = VList{sout, last_count(ex, C_SCOPE), 0u};
-            nshrink++;
+        // one shrink per search: weighing against a smaller scope again
+        // would make bottom-up steps of what top-down steps do cheaper
+        if ((puf || pub) && !shrunk) {
+            nscope = last_count(ex, C_SCOPE);
+            shrunk = true;
         }
     }
 }
 
 // ---------------------------------------------------------------------
-// Hong's first update (scc_kernels.cu:124-142): FV and BV -> the SCC of the
-// first pivot p; otherwise the vertex moves to one of three sub-ranges
-// (forward only, backward only, neither: no SCC crosses them) and is
-// appended to the next live list.
+// The end of the first FW-BW (scc_kernels.cu:124-142 for Hong,
+// assignUniqueRange, :477-484, for Slota), off the nibble words in id order:
+// vertices with both visited bits are the first pivot's SCC and stay as they
+// are -- the label write maps them to Ctl::first_min, their smallest id,
+// found here -- and every other live vertex is listed for what follows, its
+// out-degree tallied.  Its class bits (forward, backward or neither) stay as
+// its range: no SCC crosses them.
 // ---------------------------------------------------------------------
 template <class Ex>
-__device__ bool ph_hong_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
+__device__ bool ph_first_update(Ex &ex, const Graph &g, const Work &w, uint32_t *Lout)
 {
-    return run_pass(ex, PH_HONG_UPDATE, [&](unsigned, unsigned nxt) {
-        const uint32_t p = key_vertex(w.pivkey[0]);
-        uint32_t mn = 0xFFFFFFFFu;   // smallest member of the pivot's SCC seen by this thread
-        for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
-            uint32_t v[4], s[4];
-            bool ok[4];
-            load_list4(src, base + 4u * lane_id(), v, ok);
-#pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                bool surv = false;
-                if (s[j] != DEAD) {
-                    if ((s[j] & FVB) && (s[j] & BVB)) {
-                        w.st[v[j]] = DEAD;
-                        w.label[v[j]] = p;
-                        mn = min(mn, v[j]);
-                    } else {
-                        w.st[v[j]] = split_class(s[j]);
-                        surv = true;
-                    }
-                }
-                bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 15);
-            }
-            count_verts_n(ex, (unsigned)ok[0] + ok[1] + ok[2] + ok[3]);
+    return run_pass(ex, PH_FIRST_UPDATE, [&](unsigned, unsigned nxt) {
+        uint32_t mn = 0xFFFFFFFFu;
+        const uint32_t nu = g.V / 32u + 1u, cu = item_group(ex, nu);
+        for (uint32_t base = ex.wid() * cu; base < nu; base += ex.nwarps() * cu) {
+            const uint32_t u = base + lane_id();
+            const bool in = lane_id() < cu && u < nu;
+            const NibUnit x = load_unit(w, in, u);
+            const uint32_t both = x.live & x.fwd & x.bwd;
+            if (both) mn = min(mn, u * 32u + (uint32_t)__ffs(both) - 1u);
+            count_verts_n(ex, in ? min(32u, g.V + 1u - u * 32u) : 0u);
+            unit_walk2(u, x.live & ~both, [&](const bool (&ok)[2], const uint32_t (&v)[2], const unsigned (&)[2]) {
+                bq_add_edges(0, (ok[0] ? __ldg(&g.Fr[v[0] + 1u]) - __ldg(&g.Fr[v[0]]) : 0u) +
+                                    (ok[1] ? __ldg(&g.Fr[v[1] + 1u]) - __ldg(&g.Fr[v[1]]) : 0u));
+                bq_pushK<2>(0, ok, v, w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 16);
+            });
         }
-        block_min_atomic(mn, w.pivkey[0] ? &w.smin[p] : w.smin);   // mn stays 0xFFFFFFFF without a pivot
-        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl);
-    });
-}
-
-// Slota: the first FW-BW's SCC is final; every other live vertex keeps
-// which of the two searches reached it as its range (no SCC crosses those)
-// and is appended to the live list of the colour peels.
-template <class Ex>
-__device__ bool ph_slota_first_update(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
-{
-    return run_pass(ex, PH_SLOTA_FIRST_UPDATE, [&](unsigned, unsigned nxt) {
-        const uint32_t p = key_vertex(w.pivkey[0]);
-        uint32_t mn = 0xFFFFFFFFu;   // smallest member of p's SCC seen by this thread
-        for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
-            uint32_t v[4], s[4];
-            bool ok[4];
-            load_list4(src, base + 4u * lane_id(), v, ok);
-#pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                bool surv = false, scc = false;
-                if (s[j] != DEAD) {
-                    if ((s[j] & FVB) && (s[j] & BVB)) { w.st[v[j]] = DEAD; w.label[v[j]] = p; scc = true; }
-                    else { w.st[v[j]] = split_class(s[j]); surv = true; }
-                }
-                mn = scc ? min(mn, v[j]) : mn;
-                bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
-                bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 16);
-            }
-            count_verts_n(ex, (unsigned)ok[0] + ok[1] + ok[2] + ok[3]);
-        }
-        block_min_atomic(mn, w.pivkey[0] ? &w.smin[p] : w.smin);   // mn stays 0xFFFFFFFF without a pivot
-        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl, &ex.lc(nxt)[C_FE]);
-    });
-}
-
-// The same update on the whole-GPU policy, where the search kept a
-// shrinking scope: members of the first SCC (both visited bits) keep that
-// mark as their state -- no later phase treats it as live, and the label
-// write maps it to the SCC's smallest member, Ctl::first_min, which every
-// CTA folds in here from the completions it saw -- so only the search's
-// final scope is walked, not every vertex the search could reach.
-template <class Ex>
-__device__ bool ph_slota_first_update_lazy(Ex &ex, const Graph &g, const Work &w, VList src, uint32_t *Lout)
-{
-    return run_pass(ex, PH_SLOTA_FIRST_UPDATE, [&](unsigned, unsigned nxt) {
-        for (uint32_t base = ex.wid() * 128u; base < src.n; base += ex.nwarps() * 128u) {
-            uint32_t v[4], s[4];
-            bool ok[4];
-            load_list4(src, base + 4u * lane_id(), v, ok);
-#pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const bool surv = s[j] != DEAD && (s[j] & (FVB | BVB)) != (FVB | BVB);
-                if (surv) w.st[v[j]] = split_class(s[j]);
-                bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
-                bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 16);
-            }
-            count_verts_n(ex, (unsigned)ok[0] + ok[1] + ok[2] + ok[3]);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0 && *cta_first_min() != 0xFFFFFFFFu) atomicMin(&ex.ctl->first_min, *cta_first_min());
+        block_min_atomic(mn, &ex.ctl->first_min);
         bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl, &ex.lc(nxt)[C_FE]);
     });
 }
@@ -894,10 +901,10 @@ __device__ bool ph_compact(Ex &ex, const Graph &g, const Work &w, VList src, uin
             bool ok[4];
             load_list4(src, base + 4u * lane_id(), v, ok);
 #pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = ok[j] ? w.st[v[j]] : DEAD;
+            for (int j = 0; j < 4; j++) s[j] = ok[j] ? nib_of(w.nb, v[j]) : 0u;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const bool surv = s[j] != DEAD;
+                const bool surv = (s[j] & NL) != 0u;
                 bq_add_edges(0, surv ? __ldg(&g.Fr[v[j] + 1u]) - __ldg(&g.Fr[v[j]]) : 0u);
                 bq_push(0, surv, v[j], w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 18);
             }
@@ -935,33 +942,18 @@ __device__ bool ph_compact(Ex &ex, const Graph &g, const Work &w, VList src, uin
 // everywhere when they have settled, and then says that v reaches its root.
 // ---------------------------------------------------------------------
 
-// Vertices a warp takes at once from a list of n: the smallest power of two
-// that still gives every warp at most one item, at most 32.  A level's time
-// is the chain of dependent accesses of its longest item, so a short list is
-// spread over all warps before lanes are filled.
-template <class Ex>
-__device__ __forceinline__ uint32_t item_group(const Ex &ex, uint32_t n)
-{
-    uint32_t s = 32u;
-    while (s > 1u && (n + (s >> 1) - 1u) / (s >> 1) <= ex.nwarps()) s >>= 1;
-    return s;
-}
-
-// Word pairs of all vertices from their states (every state word is a range
-// class or final here).
+// Word pairs of all vertices from their nibbles: the range is the class of
+// the first search.
 template <class Ex>
 __device__ bool ph_peel_init(Ex &ex, const Graph &g, const Work &w)
 {
     return run_pass(ex, PH_PEEL_INIT, [&](unsigned, unsigned) {
         for (uint32_t i0 = ex.tid() * 2u; i0 <= g.V; i0 += ex.nthr() * 2u) {
-            const bool two = i0 + 1u <= g.V;
-            uint2 s = make_uint2(DEAD, DEAD);
-            if (two) s = *reinterpret_cast<const uint2 *>(w.st + i0);
-            else s.x = w.st[i0];
-            const bool la = (s.x & (FVB | BVB)) == 0u && s.x != DEAD, lb = (s.y & (FVB | BVB)) == 0u && s.y != DEAD;
-            const uint4 o = make_uint4(la ? s.x : FULL, la ? (i0 << 1) | 1u : FULL, lb ? s.y : FULL,
+            const uint32_t x = w.nb[i0 >> 3] >> (4u * (i0 & 7u)), ca = x & NCLASS, cb = (x >> 4) & NCLASS;
+            const bool la = (ca & NL) && ca != NCLASS, lb = (cb & NL) && cb != NCLASS;
+            const uint4 o = make_uint4(la ? ca : FULL, la ? (i0 << 1) | 1u : FULL, lb ? cb : FULL,
                                        lb ? ((i0 + 1u) << 1) | 1u : FULL);
-            if (two) *reinterpret_cast<uint4 *>(w.pc + i0) = o;
+            if (i0 + 1u <= g.V) *reinterpret_cast<uint4 *>(w.pc + i0) = o;
             else w.pc[i0] = make_uint2(o.x, o.y);
         }
     });
@@ -983,8 +975,9 @@ __device__ __forceinline__ void peel_raise2(Ex &ex, const Graph &g, const Work &
     const uint32_t o0 = t0 ? atomicMax(&w.pc[n0].y, w0) : FULL;
     const uint32_t o1 = t1 ? atomicMax(&w.pc[n1].y, w1) : FULL;
     // whoever sets the flag lists the vertex
-    bq_push(0, !(o0 & 1u) && o0 < w0, n0, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 14);
-    bq_push(0, !(o1 & 1u) && o1 < w1, n1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 14);
+    const bool push[2] = {!(o0 & 1u) && o0 < w0, !(o1 & 1u) && o1 < w1};
+    const uint32_t n[2] = {n0, n1};
+    bq_pushK<2>(0, push, n, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 14);
 }
 
 // Two arcs per lane: neighbour n joins the SCC of colour c's root.
@@ -998,8 +991,59 @@ __device__ __forceinline__ void peel_join2(Ex &ex, const Graph &g, const Work &w
     const bool t1 = v1 && w.pc[n1].y == c1 << 1;
     const uint32_t o0 = t0 ? atomicOr(&w.pc[n0].y, 1u) : 1u;
     const uint32_t o1 = t1 ? atomicOr(&w.pc[n1].y, 1u) : 1u;
-    bq_push(0, !(o0 & 1u), n0, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 13);
-    bq_push(0, !(o1 & 1u), n1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 13);
+    const bool push[2] = {!(o0 & 1u), !(o1 & 1u)};
+    const uint32_t n[2] = {n0, n1};
+    bq_pushK<2>(0, push, n, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 13);
+}
+
+// Vertices of a peel's work list, one per lane, expanded over (R, C); with
+// seeds the list is the live list (JOIN: only the roots of their colours
+// are expanded).
+template <bool RAISE, class Ex>
+__device__ __forceinline__ void peel_expand(Ex &ex, const Graph &g, const Work &w, const uint32_t *__restrict__ R,
+                                            const uint32_t *__restrict__ C, bool valid, uint32_t v, bool seeds,
+                                            unsigned par, unsigned nxt)
+{
+    uint32_t r = 0, c = 0, beg = 0, deg = 0;
+    bool act = valid;
+    if (valid) {
+        beg = __ldg(&R[v]);
+        deg = __ldg(&R[v + 1u]) - beg;
+        if (RAISE) {
+            r = w.pc[v].x;
+            c = atomicAnd(&w.pc[v].y, ~1u) >> 1;   // off the list: the newest colour
+        } else {
+            const uint32_t y = w.pc[v].y;
+            c = y >> 1;
+            if (seeds) {   // the root of its colour?
+                act = y == v << 1;
+                if (act) {
+                    w.pc[v].y = y | 1u;
+                    w.smin[v] = v;   // v represents its SCC: the update folds the members in
+                }
+            }
+        }
+    }
+    if (!RAISE && seeds) {
+        const unsigned m = __ballot_sync(FULL, act);
+        if (lane_id() == 0 && m) atomicAdd(&ex.ctl->n_pivot, (unsigned long long)__popc(m));
+        if (m == 0u) return;
+    }
+    if (!act) deg = 0u;
+    const bool heavy = deg > HEAVY_T;
+    warp_push_chunks(v, heavy ? (deg + CH - 1u) / CH : 0u, w.H[0][par], &ex.lc(nxt)[C_FH], w.hcap, ex.ctl);
+    if (heavy) deg = 0u;
+    count_verts(ex, valid);
+    auto fn = [&](bool v0, uint32_t n0, uint32_t l0, bool v1, uint32_t n1, uint32_t l1) {
+        const uint32_t c0 = __shfl_sync(FULL, c, l0), c1 = __shfl_sync(FULL, c, l1);
+        if (RAISE) {
+            const uint32_t r0 = __shfl_sync(FULL, r, l0), r1 = __shfl_sync(FULL, r, l1);
+            peel_raise2(ex, g, w, v0, n0, r0, c0, v1, n1, r1, c1, par, nxt);
+        } else {
+            peel_join2(ex, g, w, v0, n0, c0, v1, n1, c1, par, nxt);
+        }
+    };
+    count_edges(ex, lbs_walk2(beg, deg, C, fn));
 }
 
 // One fixpoint of a peel over (R, C): with RAISE the colours of the live
@@ -1015,63 +1059,28 @@ __device__ bool ph_peel_spread(Ex &ex, const Graph &g, const Work &w, VList L, c
         const bool ok = run_pass(ex, RAISE ? PH_PROP : PH_PEEL_SCC, [&](unsigned, unsigned nxt) {
             const unsigned par = ex.gl & 1u, cp = par ^ 1u;
             const uint32_t *src = lev == 0u ? L.p : w.Q[0][cp];
-            const uint32_t gs = item_group(ex, nq);
-            const uint32_t ng = (nq + gs - 1u) / gs;
+            const uint32_t gsh = item_shift(ex, nq), ng = (nq + (1u << gsh) - 1u) >> gsh;
             for (uint32_t it = ex.wid(); it < nh + ng; it += ex.nwarps()) {
                 if (it < nh) {
                     const uint2 hc = w.H[0][cp][it];
                     const uint2 x = make_uint2(vld(&w.pc[hc.x].x), vld(&w.pc[hc.x].y));
                     const uint32_t c = x.y >> 1;
-                    auto fn = [&](bool v0, uint32_t n0, uint32_t, bool v1, uint32_t n1, uint32_t) {
+                    auto fn = [&](bool v0, uint32_t n0, bool v1, uint32_t n1) {
                         if (RAISE) peel_raise2(ex, g, w, v0, n0, x.x, c, v1, n1, x.x, c, par, nxt);
                         else peel_join2(ex, g, w, v0, n0, c, v1, n1, c, par, nxt);
                     };
-                    chunk_expand(ex, R, C, hc, 0u, fn);
+                    chunk_expand(ex, R, C, hc, fn);
                     continue;
                 }
-                const uint32_t i = (it - nh) * gs + lane_id();
-                const bool valid = lane_id() < gs && i < nq;
-                const uint32_t v = valid ? src[i] : 0u;
-                uint32_t r = 0, c = 0, beg = 0, deg = 0;
-                bool act = valid;
-                if (valid) {
-                    beg = __ldg(&R[v]);
-                    deg = __ldg(&R[v + 1u]) - beg;
-                    if (RAISE) {
-                        r = w.pc[v].x;
-                        c = atomicAnd(&w.pc[v].y, ~1u) >> 1;   // off the list: the newest colour
-                    } else {
-                        const uint32_t y = w.pc[v].y;
-                        c = y >> 1;
-                        if (lev == 0u) {   // the root of its colour?
-                            act = y == v << 1;
-                            if (act) {
-                                w.pc[v].y = y | 1u;
-                                w.smin[v] = v;   // v represents its SCC: the update folds the members in
-                            }
-                        }
-                    }
-                }
-                if (!RAISE && lev == 0u) {
-                    const unsigned m = __ballot_sync(FULL, act);
-                    if (lane_id() == 0 && m) atomicAdd(&ex.ctl->n_pivot, (unsigned long long)__popc(m));
-                    if (m == 0u) continue;
-                }
-                if (!act) deg = 0u;
-                const bool heavy = deg > HEAVY_T;
-                warp_push_chunks(v, heavy ? (deg + CH - 1u) / CH : 0u, w.H[0][par], &ex.lc(nxt)[C_FH], w.hcap, ex.ctl);
-                if (heavy) deg = 0u;
-                count_verts(ex, valid);
-                auto fn = [&](bool v0, uint32_t n0, uint32_t l0, bool v1, uint32_t n1, uint32_t l1) {
-                    const uint32_t c0 = __shfl_sync(FULL, c, l0), c1 = __shfl_sync(FULL, c, l1);
-                    if (RAISE) {
-                        const uint32_t r0 = __shfl_sync(FULL, r, l0), r1 = __shfl_sync(FULL, r, l1);
-                        peel_raise2(ex, g, w, v0, n0, r0, c0, v1, n1, r1, c1, par, nxt);
-                    } else {
-                        peel_join2(ex, g, w, v0, n0, c0, v1, n1, c1, par, nxt);
-                    }
-                };
-                count_edges(ex, lbs_walk2(beg, deg, C, fn));
+                const uint32_t i = ((it - nh) << gsh) + lane_id();
+                const bool valid = lane_id() >> gsh == 0u && i < nq;
+                peel_expand<RAISE>(ex, g, w, R, C, valid, valid ? src[i] : 0u, lev == 0u, par, nxt);
+            }
+            for (unsigned left = Ex::grid ? PEEL_ROUNDS : 0u; left; left--) {
+                uint32_t v;
+                const unsigned took = bq_pop(0, w.qcap, 1u, local_cap(w.qcap), v);
+                if (took == 0u) break;
+                peel_expand<RAISE>(ex, g, w, R, C, lane_id() < took, v, false, par, nxt);
             }
             bq_flush(1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], nullptr, nullptr, g.V, ex.ctl);
         });
@@ -1100,7 +1109,6 @@ __device__ bool ph_peel_update(Ex &ex, const Graph &g, const Work &w, VList src,
                 const uint32_t c = y[j] >> 1;
                 if (scc) {
                     w.pc[v[j]] = make_uint2(FULL, FULL);
-                    w.st[v[j]] = DEAD;
                     w.label[v[j]] = c;
                 }
                 if (surv) w.pc[v[j]] = make_uint2(c, (v[j] << 1) | 1u);
@@ -1137,9 +1145,8 @@ enum { RUN_DONE = 0, RUN_SWITCH = 1, RUN_RESIDUAL = 2, RUN_ERROR = -1 };
 // reference counts each SCC its main loop / colouring finds once
 // (scc_WCC.cu:933-949, scc_Coloring.cu:640-652), so the counters and the
 // canonical labels are those of any complete run.
-//   pass 1 (all CTAs): live vertex L[i] gets the state word FV|BV|(i + 1)
-//          (at a loop head the only other vertices with both bits are the
-//          first SCC's members, marked FV|BV|0);
+//   pass 1 (all CTAs): live vertex L[i] gets its local number i and the
+//          residual flag in its nibble;
 //   pass 2 (all CTAs): the arcs between live vertices, as (i << 16) | j,
 //          into a work queue;
 //   then one CTA loads them into shared memory and peels SCCs by colour
@@ -1207,7 +1214,10 @@ __device__ bool res_extract(Ex &ex, const Graph &g, const Work &w, Carry &cy)
     const uint32_t *L = w.L[cy.lsel];
     const uint32_t n = cy.nL;
     if (!run_pass(ex, PH_RES_TAG, [&](unsigned, unsigned) {
-            for (uint32_t i = ex.tid(); i < n; i += ex.nthr()) w.st[L[i]] = FVB | BVB | (i + 1u);
+            for (uint32_t i = ex.tid(); i < n; i += ex.nthr()) {
+                w.st[L[i]] = i;
+                nib_or(w.nb, L[i], NQ);
+            }
         }))
         return false;
     const bool ok = run_pass(ex, PH_RES_EXTRACT, [&](unsigned, unsigned nxt) {
@@ -1217,17 +1227,16 @@ __device__ bool res_extract(Ex &ex, const Graph &g, const Work &w, Carry &cy)
             const bool valid = i < n;
             const uint32_t v = valid ? L[i] : 0u;
             const uint32_t beg = valid ? __ldg(&g.Fr[v]) : 0u, deg = valid ? __ldg(&g.Fr[v + 1u]) - beg : 0u;
-            const uint32_t r = valid && cy.peels ? w.pc[v].x : 0u;
+            const uint32_t r = !valid ? 0u : cy.peels ? w.pc[v].x : nib_of(w.nb, v) & NCLASS;
             auto fn = [&](bool ok2, uint32_t u, uint32_t own) {
                 bool hit = false;
                 uint32_t e = 0;
                 const uint32_t src = __shfl_sync(FULL, i, own), rs = __shfl_sync(FULL, r, own);
                 if (ok2) {
                     u = guard_id(u, g.V, ex.ctl);
-                    const uint32_t s = w.st[u];
-                    // live vertex i carries FV|BV|(i + 1); FV|BV|0 marks the first SCC's members
-                    hit = (s & (FVB | BVB)) == (FVB | BVB) && (s & RMASK) != 0u && (!cy.peels || w.pc[u].x == rs);
-                    e = (src << 16) | ((s & RMASK) - 1u);
+                    const uint32_t x = nib_of(w.nb, u);
+                    hit = (x & (NL | NQ)) == (NL | NQ) && (cy.peels ? w.pc[u].x : x & NCLASS) == rs;
+                    if (hit) e = (src << 16) | w.st[u];
                 }
                 warp_push(hit, e, eb, &ex.lc(nxt)[C_BQ], RES_MAX_E, ex.ctl, 24);
             };
@@ -1240,13 +1249,13 @@ __device__ bool res_extract(Ex &ex, const Graph &g, const Work &w, Carry &cy)
 
 // The solver (every thread of one CTA).  L[0..n): the live vertices;
 // eb[0..m): their arcs (i << 16) | j.  Writes every live vertex's
-// canonical label (LBL_SELF: the smallest id of its SCC) and DEAD state, and
-// adds the SCCs found to n_pivot.  Each peel removes at least the root with
+// canonical label (LBL_SELF: the smallest id of its SCC) and adds the SCCs
+// found to n_pivot.  Each peel removes at least the root with
 // the largest (or smallest) key, so at most n peels, each with at most n + 1
 // sweeps per fixpoint.
-// With out set the canonical labels of the residual vertices go straight to
-// out and their state words keep the residual tag: the other CTAs are
-// writing every other vertex's label meanwhile, deciding by that tag.
+// With out set the canonical labels of the residual vertices also go straight
+// to out: the other CTAs are writing every other vertex's label meanwhile,
+// leaving out those with the residual flag.
 static __device__ __noinline__ void res_solve(const Graph &g, const Work &w, const uint32_t *L, uint32_t n, const uint32_t *eb,
                           uint32_t m, Ctl *ctl, uint32_t *out = nullptr)
 {
@@ -1352,7 +1361,6 @@ static __device__ __noinline__ void res_solve(const Graph &g, const Work &w, con
     for (uint32_t i = t; i < n; i += T) {
         w.label[gid[i]] = LBL_SELF | aux[col[i]];
         if (out) out[gid[i] - 1u] = aux[col[i]];
-        else w.st[gid[i]] = DEAD;
     }
     if (t == 0) {
         atomicAdd(&ctl->n_pivot, (unsigned long long)s_npiv);
@@ -1387,7 +1395,7 @@ __device__ int residual(Ex &ex, const Graph &g, const Work &w, Carry &cy)
 }
 
 // Colour peels until no vertex is left.  Entry: live list L[lsel] with nL
-// entries, nE out-arcs, their ranges in the state words.
+// entries, nE out-arcs, their ranges in the nibbles.
 template <class Ex>
 __device__ int peel_loop(Ex &ex, const Graph &g, const Work &w, Carry &cy, uint32_t tail_n)
 {
@@ -1412,37 +1420,23 @@ __device__ int peel_loop(Ex &ex, const Graph &g, const Work &w, Carry &cy, uint3
     return RUN_DONE;
 }
 
-// First pivot over the live vertices after trim1 to fixpoint
-// (pollForFirstPivot / selectFirstPivot, scc_WCC.cu:701-703); the live
-// vertices are compacted into Lout on the way.
+// The pivot over the live vertices after trim1 to its fixpoint
+// (pollForFirstPivot / selectFirstPivot, scc_WCC.cu:701-703), into pivkey[1]:
+// run only when the pivot that the init pass found was trimmed since (else
+// it is still the largest).
 template <class Ex>
-__device__ bool ph_first_pivot(Ex &ex, const Graph &g, const Work &w, uint32_t *Lout)
+__device__ bool ph_first_pivot(Ex &ex, const Graph &g, const Work &w)
 {
-    return run_pass(ex, PH_FIRST_PIVOT, [&](unsigned, unsigned nxt) {
+    return run_pass(ex, PH_FIRST_PIVOT, [&](unsigned, unsigned) {
         unsigned long long best = 0;
-        for (uint32_t base = ex.wid() * 128u; base <= g.V; base += ex.nwarps() * 128u) {
-            const uint32_t i0 = base + 4u * lane_id();
-            uint32_t st4[4] = {DEAD, DEAD, DEAD, DEAD};
-            if (i0 + 3u <= g.V) {
-                const uint4 x = *reinterpret_cast<const uint4 *>(w.st + i0);
-                st4[0] = x.x; st4[1] = x.y; st4[2] = x.z; st4[3] = x.w;
-            } else {
-                for (uint32_t j = 0; j < 4u && i0 + j <= g.V; j++) st4[j] = w.st[i0 + j];
+        const uint32_t nwords = g.V / 8u + 1u;
+        for (uint32_t wd = ex.tid(); wd < nwords; wd += ex.nthr()) {
+            for (uint32_t m = w.nb[wd] & NIBS; m; m &= m - 1u) {
+                const unsigned long long k = pivot_key(g, wd * 8u + ((uint32_t)__ffs(m) - 1u) / 4u);
+                best = k > best ? k : best;
             }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint32_t v = i0 + (uint32_t)j;
-                const bool live = v >= 1u && v <= g.V && st4[j] != DEAD;
-                if (live) {
-                    unsigned long long k = pivot_key(g, v);
-                    best = k > best ? k : best;
-                }
-                bq_push(0, live, v, w.qcap, Lout, &ex.lc(nxt)[C_LIST], g.V, ex.ctl, 20);
-            }
-            count_verts_n(ex, i0 <= g.V ? min(4u, g.V + 1u - i0) : 0u);
         }
-        block_max_atomic(best, &w.pivkey[0]);
-        bq_flush(1, w.qcap, Lout, &ex.lc(nxt)[C_LIST], nullptr, nullptr, g.V, ex.ctl);
+        block_max_atomic(best, &w.pivkey[1]);
     });
 }
 
@@ -1451,69 +1445,59 @@ __device__ __forceinline__ unsigned long long vld64(const unsigned long long *p)
     return *(const volatile unsigned long long *)p;
 }
 
-// The first FW-BW of every driver, from the single pivot in pivkey[0]
-// (scc_WCC.cu:717-743, scc_Coloring.cu:539-565; wHong / wSlota run it with
-// the virtual-warp schedule, scc_WCC.cu:209-317, scc_Coloring.cu:154-263).
-template <class Ex>
-__device__ bool first_fwbw(Ex &ex, const Graph &g, const Work &w, int lw, VList scope, VList *last = nullptr)
-{
-    const unsigned long long k = vld64(&w.pivkey[0]);
-    if (k == 0ull) return true;   // no live vertex
-    return ph_bfs(ex, g, w, key_vertex(k), lw, scope, last);
-}
-
-// vHong / wHong up to the main loop (scc_WCC.cu:573-848): trim1*, first
-// pivot, FW-BW, update, trim1*, trim2, trim1*, live list of what is left.
+// vHong / wHong up to the peels (scc_WCC.cu:573-848): trim1*, first pivot,
+// FW-BW, update, trim1*, trim2, trim1*, live list of what is left.  wHong /
+// wSlota run the FW-BW with the virtual-warp schedule (scc_WCC.cu:209-317,
+// scc_Coloring.cu:154-263).
 template <class Ex>
 __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t2, int lw, Carry &cy)
 {
-    const VList all{nullptr, g.V, 1u};
-    VList scope = all;
-    if (!ph_init(ex, g, w, !t1)) return RUN_ERROR;
-    if (t1) {
-        if (!ph_trim1_fix(ex, g, w, all, true)) return RUN_ERROR;
-        if (!ph_first_pivot(ex, g, w, w.L[0])) return RUN_ERROR;
-        scope = VList{w.L[0], last_count(ex, C_LIST), 0u};
+    if (!ph_init(ex, g, w, t1, t1)) return RUN_ERROR;
+    uint32_t nlive = last_count(ex, C_LIST);
+    unsigned long long k = vld64(&w.pivkey[0]);
+    if (t1 && nlive) {
+        if (!ph_trim1_fix(ex, g, w, VList{nullptr, nlive, 0u}, true)) return RUN_ERROR;
+        nlive = g.V - (uint32_t)vld64(&ex.ctl->n_trim1);
+        if (nlive && !(nib_of(w.nb, key_vertex(k)) & NL)) {
+            if (!ph_first_pivot(ex, g, w)) return RUN_ERROR;
+            k = vld64(&w.pivkey[1]);
+        }
     }
-    if (!first_fwbw(ex, g, w, lw, scope)) return RUN_ERROR;
-    if (!ph_hong_update(ex, g, w, scope, w.L[1])) return RUN_ERROR;
+    cy.gl = ex.gl;
+    if (nlive == 0u) return RUN_DONE;
+    if (!ph_bfs(ex, g, w, key_vertex(k), lw, nlive)) return RUN_ERROR;
+    if (!ph_first_update(ex, g, w, w.L[1])) return RUN_ERROR;
     const VList L1{w.L[1], last_count(ex, C_LIST), 0u};
     cy.gl = ex.gl;
     if (L1.n == 0u) return RUN_DONE;   // every vertex is trimmed or in the first SCC
+    cy.lsel = 1u;
+    cy.nL = L1.n;
+    cy.nE = last_count(ex, C_FE);
     if (t1 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
     if (t2 && !ph_trim2(ex, g, w, L1)) return RUN_ERROR;
     if (t1 && t2 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
-    if (!ph_compact(ex, g, w, L1, w.L[0])) return RUN_ERROR;
-    cy.lsel = 0u;
-    cy.nL = last_count(ex, C_LIST);
-    cy.nE = last_count(ex, C_FE);
+    if (t1 || t2) {
+        if (!ph_compact(ex, g, w, L1, w.L[0])) return RUN_ERROR;
+        cy.lsel = 0u;
+        cy.nL = last_count(ex, C_LIST);
+        cy.nE = last_count(ex, C_FE);
+    }
     cy.gl = ex.gl;
     return RUN_DONE;
 }
 
-// vSlota / wSlota up to the colouring loop (scc_Coloring.cu:403-587):
-// trim1 once, first pivot, FW-BW, update.  t2 is not used by the
-// reference's Slota drivers.
+// vSlota / wSlota up to the peels (scc_Coloring.cu:403-587): trim1 once,
+// first pivot, FW-BW, update.  t2 is not used by the reference's Slota
+// drivers.
 template <class Ex>
 __device__ int slota_front(Ex &ex, const Graph &g, const Work &w, bool t1, int lw, Carry &cy)
 {
-    VList scope{nullptr, g.V, 1u};
-    if (t1) {
-        if (!ph_init_trim1(ex, g, w, w.L[0])) return RUN_ERROR;
-        scope = VList{w.L[0], last_count(ex, C_LIST), 0u};
-    } else if (!ph_init(ex, g, w, true)) {
-        return RUN_ERROR;
-    }
-    if constexpr (Ex::nbq > 2) {
-        // whole GPU: the first SCC's members keep their FV|BV mark and the
-        // update walks only the search's final, shrunken scope
-        VList last = scope;
-        if (!first_fwbw(ex, g, w, lw, scope, &last)) return RUN_ERROR;
-        if (!ph_slota_first_update_lazy(ex, g, w, last, w.L[1])) return RUN_ERROR;
-    } else {
-        if (!first_fwbw(ex, g, w, lw, scope)) return RUN_ERROR;
-        if (!ph_slota_first_update(ex, g, w, scope, w.L[1])) return RUN_ERROR;
-    }
+    if (!ph_init(ex, g, w, t1, false)) return RUN_ERROR;
+    const uint32_t nlive = last_count(ex, C_LIST);
+    cy.gl = ex.gl;
+    if (nlive == 0u) return RUN_DONE;
+    if (!ph_bfs(ex, g, w, key_vertex(vld64(&w.pivkey[0])), lw, nlive)) return RUN_ERROR;
+    if (!ph_first_update(ex, g, w, w.L[1])) return RUN_ERROR;
     cy.lsel = 1u;
     cy.nL = last_count(ex, C_LIST);
     cy.nE = last_count(ex, C_FE);
