@@ -785,7 +785,8 @@ __device__ __forceinline__ unsigned lbs_walk2(uint32_t beg, uint32_t deg, const 
     return total;
 }
 
-// Same walk, four entries per lane per step: fn(valid[4], neighbour[4]).
+// Same walk, four entries per lane per step: fn(valid[4], neighbour[4],
+// owner's lane[4]).
 template <class Fn>
 __device__ __forceinline__ unsigned lbs_walk4(uint32_t beg, uint32_t deg, const uint32_t *__restrict__ C, Fn &&fn)
 {
@@ -794,6 +795,7 @@ __device__ __forceinline__ unsigned lbs_walk4(uint32_t beg, uint32_t deg, const 
     for (unsigned base = 0; base < total; base += 128u) {
         bool ok[4];
         uint32_t n[4];
+        unsigned own[4];
 #pragma unroll
         for (unsigned j = 0; j < 4u; j++) {
             const unsigned e = base + 32u * j + lane_id();
@@ -806,8 +808,9 @@ __device__ __forceinline__ unsigned lbs_walk4(uint32_t beg, uint32_t deg, const 
             const uint32_t a = __shfl_sync(FULL, at, lo);
             ok[j] = e < total;
             n[j] = ok[j] ? __ldg(&C[a + e]) : 0u;
+            own[j] = lo;
         }
-        fn(ok, n);
+        fn(ok, n, own);
     }
     return total;
 }
