@@ -140,6 +140,8 @@ __host__ __device__ constexpr size_t nib_bytes(size_t V) { return ((V / 8 + 1) *
 // (nullptr: only count).  Returns the bytes used.  Same layout on host and
 // device; used by the batched form, where every CTA re-carves its private
 // scratch for each graph it takes.
+// A chunk queue holds one cut of every vertex above HEAVY_T (at most deg / CH + 1
+// chunks each): no pass may cut a vertex twice.
 __host__ __device__ inline size_t carve_work(char *base, uint32_t V, uint32_t E, Work *w)
 {
     const size_t n1 = (size_t)V + 1;

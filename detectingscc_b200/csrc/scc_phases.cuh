@@ -992,17 +992,28 @@ __device__ __forceinline__ void peel_visit(Ex &ex, const Graph &g, const Work &w
 
 // Vertices of a peel's work list, one per lane, expanded over (R, C); with
 // seeds the list is the live list (JOIN: only the roots of their colours
-// are expanded).
+// are expanded).  local: v comes off the warp's own slice.  A raised vertex
+// can come off slices again and again within a pass, and the chunk queues
+// have room for one cut of every heavy vertex; so a heavy one taken off a
+// slice is not cut but goes, with its flag still set (nobody lists it again),
+// to the next pass.  JOIN takes every vertex once.
 template <bool RAISE, class Ex>
 __device__ __forceinline__ void peel_expand(Ex &ex, const Graph &g, const Work &w, const uint32_t *__restrict__ R,
                                             const uint32_t *__restrict__ C, bool valid, uint32_t v, bool seeds,
-                                            unsigned par, unsigned nxt)
+                                            unsigned par, unsigned nxt, bool local = false)
 {
     uint32_t r = 0, c = 0, beg = 0, deg = 0;
     bool act = valid;
     if (valid) {
         beg = __ldg(&R[v]);
         deg = __ldg(&R[v + 1u]) - beg;
+    }
+    if (RAISE && local) {
+        const bool later = deg > HEAVY_T;
+        warp_push(later, v, w.Q[0][par], &ex.lc(nxt)[C_FQ], g.V, ex.ctl, 15);
+        if (later) valid = act = false;
+    }
+    if (valid) {
         if (RAISE) {
             r = w.pc[v].x;
             c = atomicAnd(&w.pc[v].y, ~1u) >> 1;   // off the list: the newest colour
@@ -1081,7 +1092,7 @@ __device__ bool ph_peel_spread(Ex &ex, const Graph &g, const Work &w, VList L, c
                 uint32_t v;
                 const unsigned took = bq_pop(0, w.qcap, 1u, local_cap(w.qcap), v);
                 if (took == 0u) break;
-                peel_expand<RAISE>(ex, g, w, R, C, lane_id() < took, v, false, par, nxt);
+                peel_expand<RAISE>(ex, g, w, R, C, lane_id() < took, v, false, par, nxt, true);
             }
             bq_flush(1, w.qcap, w.Q[0][par], &ex.lc(nxt)[C_FQ], nullptr, nullptr, g.V, ex.ctl);
         });
