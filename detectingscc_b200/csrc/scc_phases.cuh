@@ -58,6 +58,11 @@ __device__ __forceinline__ void count_verts_n(Ex &ex, unsigned n)
     }
 }
 
+// Passes that a search or a spread of colours can take: at most V hops, each
+// one pass, or two where the vertex is heavy (one cuts its list, the next
+// walks the chunks).
+__device__ __forceinline__ uint32_t max_levels(uint32_t V) { return 2u * V + 4u; }
+
 // Vertices a warp takes at once from a list of n (1 << item_shift): the smallest power of two
 // that still gives every warp at most one item, at most 32.  A level's time
 // is the chain of dependent accesses of its longest item, so a short list is
@@ -758,7 +763,7 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
         const uint32_t nf = last_count(ex, C_FQ), nb = last_count(ex, C_BQ);
         const uint32_t nhf = last_count(ex, C_FH), nhb = last_count(ex, C_BH);
         if (nf + nb + nhf + nhb == 0u) return true;
-        if (lev > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 40); return false; }
+        if (lev > max_levels(g.V)) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 40); return false; }
         // Beamer's rule: bottom-up when the frontier has more edges to
         // expand than the scope has vertices to test (times bu_k)
         const uint32_t mf = last_count(ex, C_FE), mb = last_count(ex, C_BE);
@@ -1061,7 +1066,7 @@ __device__ bool ph_peel_spread(Ex &ex, const Graph &g, const Work &w, VList L, c
 {
     uint32_t nq = L.n, nh = 0;
     for (unsigned lev = 0;; lev++) {
-        if (lev > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, RAISE ? 50 : 40); return false; }
+        if (lev > max_levels(g.V)) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, RAISE ? 50 : 40); return false; }
         const bool ok = run_pass(ex, RAISE ? PH_PROP : PH_PEEL_SCC, [&](unsigned, unsigned nxt) {
             const unsigned par = ex.gl & 1u, cp = par ^ 1u;
             const uint32_t *src = lev == 0u ? L.p : w.Q[0][cp];
