@@ -106,6 +106,25 @@ __device__ __forceinline__ uint32_t local_cap(uint32_t qcap, bool full = false)
     return full && qcap > 256u ? qcap - 128u : min(96u, qcap / 2u);
 }
 
+// Where they do not (spreads): a search that grows fast has few levels to
+// merge, and a warp that goes on with its finds runs past the level that would
+// go bottom-up and walks, top-down and on its own, what all would share.
+// fwd, bwd: arcs of the next level, if all but one arc a vertex of this one
+// find a new vertex; grow: arcs a vertex less one.  A pass stays one level
+// when the next is work for every warp and the one after it would be
+// bottom-up (batched graphs, whose passes are cheaper: a quarter of that).
+// Random graphs, 2M vertices of degree 5 and 12, vSlota: 495 -> 290 and
+// 309 -> 224 us; one CTA, 8,000 of degree 8: 159 -> 98 us; 600 of up to 4,096
+// of degree 12 at once: 249 -> 143 us.  grow is 2.4 on the grids and their
+// passes stay long.
+constexpr float SPREAD_ARCS = 256.0f;   // of a level, a warp: two steps of a walk
+template <class Ex>
+__device__ __forceinline__ bool spreads(const Ex &ex, float fwd, float bwd, float grow, float bottom_up)
+{
+    return fwd + bwd > SPREAD_ARCS * (float)ex.nwarps() &&
+           fmaxf(fwd, bwd) * grow > (Ex::grid ? bottom_up : 0.25f * bottom_up);
+}
+
 // Bits 0, 4, ..., 28 of a nibble word as bits 0 .. 7.
 __device__ __forceinline__ uint32_t nib8(uint32_t m)
 {
@@ -726,6 +745,9 @@ template <class Ex>
 __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw, uint32_t nscope)
 {
     bool shrunk = false;
+    const float degree = (float)g.E / (float)g.V, grow = fmaxf(degree - 1.0f, 0.0f);
+    const bool wide = w.bu_k && 2.0f * (float)nscope * grow > SPREAD_ARCS * (float)ex.nwarps();   // spreads() can hold
+    uint32_t rest = nscope;   // live vertices still unvisited in some direction, as of the last bottom-up step
     bool ok = run_pass(ex, PH_BFS0, [&](unsigned, unsigned nxt) {
         const unsigned par = ex.gl & 1u;
         if (ex.leader()) {
@@ -772,6 +794,14 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
         const uint32_t mf = last_count(ex, C_FE), mb = last_count(ex, C_BE);
         const bool puf = w.bu_k && (unsigned long long)mf > (unsigned long long)nscope * w.bu_k;
         const bool pub = w.bu_k && (unsigned long long)mb > (unsigned long long)nscope * w.bu_k;
+        // may warps go on with their own finds?
+        bool local = lw < 0;
+        if (local && wide) {
+            const float xf = (known & 1u ? (float)mf : (float)nf * degree) + (float)(nhf * CH);
+            const float xb = (known & 2u ? (float)mb : (float)nb * degree) + (float)(nhb * CH);
+            local = !spreads(ex, fminf(xf, (float)rest) * grow, fminf(xb, (float)rest) * grow, grow,
+                             (float)nscope * (float)w.bu_k);
+        }
         unsigned cm = 3u;   // bit d: this pass tallies direction d
         if constexpr (Ex::grid) {
             cm = 0u;
@@ -839,7 +869,7 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
                     bfs_expand_vwk(ex, g, w, dir, vk, ak, lw, par, nxt, (cm >> dir) & 1u);
                 }
             }
-            if (lw < 0) {
+            if (local) {
                 for (int dir = 0; dir < 2; dir++) {
                     if (dir ? pub : puf) continue;   // found bottom-up: left to the next pass
                     uint32_t edges = 0;
@@ -858,8 +888,9 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
         if (!ok) return false;
         // one shrink per search: weighing against a smaller scope again
         // would make bottom-up steps of what top-down steps do cheaper
-        if ((puf || pub) && !shrunk) {
-            nscope = last_count(ex, C_SCOPE);
+        if (puf || pub) {
+            rest = last_count(ex, C_SCOPE);
+            if (!shrunk) nscope = rest;
             shrunk = true;
         }
     }
