@@ -8,20 +8,17 @@
 
 namespace sccb {
 
-// A vertex list: p[0..n) or, with p == nullptr, the implicit list
-// base, base+1, ..., base+n-1.
+// A vertex list.
 struct VList {
     const uint32_t *p;
     uint32_t n;
-    uint32_t base;
-    __device__ __forceinline__ uint32_t at(uint32_t i) const { return p ? p[i] : base + i; }
 };
 
 // Four consecutive entries of a list for this lane (entries i0 .. i0+3): one
-// 128-bit load for explicit lists (list buffers are 256-byte aligned).
+// 128-bit load (list buffers are 256-byte aligned).
 __device__ __forceinline__ void load_list4(const VList &src, uint32_t i0, uint32_t (&v)[4], bool (&ok)[4])
 {
-    if (src.p && i0 + 3u < src.n) {
+    if (i0 + 3u < src.n) {
         const uint4 x = *reinterpret_cast<const uint4 *>(src.p + i0);
         v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
         ok[0] = ok[1] = ok[2] = ok[3] = true;
@@ -30,7 +27,7 @@ __device__ __forceinline__ void load_list4(const VList &src, uint32_t i0, uint32
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         ok[j] = i0 + (uint32_t)j < src.n;
-        v[j] = ok[j] ? src.at(i0 + (uint32_t)j) : 0u;
+        v[j] = ok[j] ? src.p[i0 + (uint32_t)j] : 0u;
     }
 }
 
@@ -99,7 +96,7 @@ __device__ __forceinline__ uint32_t item_group(const Ex &ex, uint32_t n)
 // to the global queue and are spread over all warps by the next pass.
 // Until there is work for every warp (full) only short slices stay: a warp
 // whose slice grows fast shares it.
-constexpr uint32_t LOCAL_ROUNDS = 16, FULL_ROUNDS = 16, LOCAL_EDGES = 4096;   // of the first search
+constexpr uint32_t LOCAL_ROUNDS = 16, LOCAL_EDGES = 4096;   // of the first search
 constexpr uint32_t PEEL_ROUNDS = 8;     // of the peels
 __device__ __forceinline__ uint32_t local_cap(uint32_t qcap, bool full = false)
 {
@@ -348,8 +345,8 @@ __device__ bool ph_init(Ex &ex, const Graph &g, const Work &w, bool trim, bool s
 
 // ---------------------------------------------------------------------
 // trim1 iterated to its fixpoint (vHong / wHong, scc_WCC.cu:680-687,
-// :773-780, :808-815).  Pass 0 checks every live vertex (all: by id, off the
-// nibble units, n of them) or a list; a trimmed vertex queues its live neighbours of the
+// :773-780, :808-815).  Pass 0 checks a list or, without one, every live
+// vertex (by id, off the nibble units); a trimmed vertex queues its live neighbours of the
 // same class for the next pass (stamped with the pass, so none is listed
 // twice; a vertex that is being checked meanwhile is listed all the same),
 // so later passes only recheck vertices that lost a neighbour.  A vertex is checked by searching both its lists for one live
@@ -411,14 +408,14 @@ __device__ __forceinline__ void trim1_check(Ex &ex, const Graph &g, const Work &
 }
 
 template <class Ex>
-__device__ bool ph_trim1_fix(Ex &ex, const Graph &g, const Work &w, VList src0, bool all)
+__device__ bool ph_trim1_fix(Ex &ex, const Graph &g, const Work &w, VList src0)
 {
     uint32_t nq = src0.n;
     for (unsigned it = 0;; it++) {
         if (it > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 30); return false; }
         const bool ok = run_pass(ex, PH_TRIM1_FIX, [&](unsigned, unsigned nxt) {
             const unsigned par = ex.gl & 1u;
-            if (all && it == 0u) {
+            if (!src0.p && it == 0u) {
                 const uint32_t nu = g.V / 32u + 1u, cu = unit_group(ex, g.V), ni = (nu + cu - 1u) / cu;
                 for (uint32_t i = ex.wid(); i < ni; i += ex.nwarps()) {
                     const uint32_t u = lane_id() * ni + i;
@@ -508,7 +505,7 @@ __device__ bool ph_trim2(Ex &ex, const Graph &g, const Work &w, VList src)
         for (uint32_t base = ex.wid() * gs; base < src.n; base += ex.nwarps() * gs) {
             uint32_t i = base + lane_id();
             bool valid = lane_id() < gs && i < src.n, hit = false, cnt = false;
-            uint32_t v = valid ? src.at(i) : 0u;
+            uint32_t v = valid ? src.p[i] : 0u;
             if (valid) {
                 const uint32_t s = nib_of(w.nb, v);
                 if (s & NL) {
@@ -873,7 +870,7 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
                 for (int dir = 0; dir < 2; dir++) {
                     if (dir ? pub : puf) continue;   // found bottom-up: left to the next pass
                     uint32_t edges = 0;
-                    for (unsigned left = full ? FULL_ROUNDS : LOCAL_ROUNDS; left && edges < LOCAL_EDGES; left--) {
+                    for (unsigned left = LOCAL_ROUNDS; left && edges < LOCAL_EDGES; left--) {
                         uint32_t v;
                         const unsigned took = bq_pop((unsigned)dir, w.qcap, full ? 24u : 1u, local_cap(w.qcap, full), v);
                         if (took == 0u) break;
@@ -1459,7 +1456,7 @@ __device__ int peel_loop(Ex &ex, const Graph &g, const Work &w, Carry &cy, uint3
         cy.paired = true;
         if (Ex::grid && cy.nL <= tail_n) { cy.gl = ex.gl; return RUN_SWITCH; }
         if (ex.leader()) ex.ctl->outer++;
-        const VList L{w.L[cy.lsel], cy.nL, 0u};
+        const VList L{w.L[cy.lsel], cy.nL};
         const bool odd = (cy.peels & 1u) != 0u;
         const uint32_t *R0 = odd ? g.Br : g.Fr, *C0 = odd ? g.Bc : g.Fc;
         const uint32_t *R1 = odd ? g.Fr : g.Br, *C1 = odd ? g.Fc : g.Bc;
@@ -1511,7 +1508,7 @@ __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t
     uint32_t nlive = last_count(ex, C_LIST);
     unsigned long long k = vld64(&w.pivkey[0]);
     if (t1 && nlive) {
-        if (!ph_trim1_fix(ex, g, w, VList{nullptr, nlive, 0u}, true)) return RUN_ERROR;
+        if (!ph_trim1_fix(ex, g, w, VList{nullptr, nlive})) return RUN_ERROR;
         nlive = g.V - (uint32_t)vld64(&ex.ctl->n_trim1);
         if (nlive && !(nib_of(w.nb, key_vertex(k)) & NL)) {
             if (!ph_first_pivot(ex, g, w)) return RUN_ERROR;
@@ -1522,15 +1519,15 @@ __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t
     if (nlive == 0u) return RUN_DONE;
     if (!ph_bfs(ex, g, w, key_vertex(k), lw, nlive)) return RUN_ERROR;
     if (!ph_first_update(ex, g, w, w.L[1])) return RUN_ERROR;
-    const VList L1{w.L[1], last_count(ex, C_LIST), 0u};
+    const VList L1{w.L[1], last_count(ex, C_LIST)};
     cy.gl = ex.gl;
     if (L1.n == 0u) return RUN_DONE;   // every vertex is trimmed or in the first SCC
     cy.lsel = 1u;
     cy.nL = L1.n;
     cy.nE = last_count(ex, C_FE);
-    if (t1 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
+    if (t1 && !ph_trim1_fix(ex, g, w, L1)) return RUN_ERROR;
     if (t2 && !ph_trim2(ex, g, w, L1)) return RUN_ERROR;
-    if (t1 && t2 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
+    if (t1 && t2 && !ph_trim1_fix(ex, g, w, L1)) return RUN_ERROR;
     if (t1 || t2) {
         if (!ph_compact(ex, g, w, L1, w.L[0])) return RUN_ERROR;
         cy.lsel = 0u;
