@@ -546,11 +546,16 @@ __device__ bool ph_trim2(Ex &ex, const Graph &g, const Work &w, VList src)
 //
 // K arcs per lane: all gathers, then all claims are issued before any
 // append.  eager (a short frontier, where a level's time is its chain of
-// dependent accesses): the claim is made without looking first -- a visited
-// bit on a vertex that is not live means nothing -- and the offsets of the
-// vertex are brought into L1 beside it, for the warp that goes on with it.  cnt (uniform over the CTA) adds the claimed vertices' degrees to
-// the pass's frontier-edge tally; a pass whose claims cannot reach the
-// bottom-up threshold skips those offset gathers.
+// dependent accesses): the claim is made without looking first, and the
+// offsets of the vertex are brought into L1 beside it, for the warp that goes
+// on with it.  This sets visited bits on trimmed vertices too.  They mean
+// nothing there: a bottom-up step takes a visited neighbour as one reached
+// through live vertices, and a trimmed vertex never lies between two live ones
+// (it has no live in-neighbour or no live out-neighbour, by its degrees or by
+// trim-1 to its fixpoint).  The step tests the live bit all the same, which
+// costs nothing.  cnt (uniform over the CTA) adds the claimed vertices'
+// degrees to the pass's frontier-edge tally; a pass whose claims are not
+// expected to reach the bottom-up threshold skips those offset gathers.
 // ---------------------------------------------------------------------
 template <int K, class Ex>
 __device__ __forceinline__ void bfs_visit(Ex &ex, const Graph &g, const Work &w, int dir, const bool (&v)[K],
@@ -698,7 +703,7 @@ __device__ __forceinline__ void bfs_pull(Ex &ex, const Graph &g, const Work &w, 
     uint32_t left = __popc(x.live & ~(x.fwd & x.bwd));
     unit_walk2(u, wf | wb, [&](const bool (&in)[2], const uint32_t (&v)[2], const unsigned (&own)[2]) {
         uint32_t pos[4], end[4];
-        const uint32_t want[4] = {NF, NB, NF, NB};
+        const uint32_t want[4] = {NL | NF, NL | NB, NL | NF, NL | NB};
         bool half[2];   // already visited the other way
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -711,7 +716,7 @@ __device__ __forceinline__ void bfs_pull(Ex &ex, const Graph &g, const Work &w, 
             pos[2 * h + 1] = nb ? __ldg(&g.Fr[v[h]]) : 0u;
             end[2 * h + 1] = nb ? __ldg(&g.Fr[v[h] + 1u]) : 0u;
         }
-        const uint32_t found = find4(ex, g, w, pos, end, NF, NB, want);
+        const uint32_t found = find4(ex, g, w, pos, end, NL | NF, NL | NB, want);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const bool ff = found >> (2 * h) & 1u, fb = found >> (2 * h + 1) & 1u;
