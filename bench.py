@@ -297,7 +297,9 @@ def run_ours(args):
     assert np.array_equal(lab_fwd, labels.cpu().numpy().view(np.uint32))
     file_leg = None if args.no_file_leg else file_to_labels(eng, hg, labels, lab_fwd, cfg, sh, world, rank, args)
 
-    B_alg = 8 * ins["edges_scanned"] + 12 * ins["vertex_visits"]
+    # T_v: the init sweep's V vertices (8 B of offsets read, half a byte written, half a byte read by the first
+    # update) and those that are visited one by one (offset, state and list entry: 12 B)
+    B_alg = 8 * ins["edges_scanned"] + 12 * (ins["vertex_visits"] - V) + 9 * V
     peak, peak_kind = _peak_hbm()
     achieved = B_alg / (t_kern * 1e-3) / 1e9
     tr = _traffic(args.config if args.scale is None else None)

@@ -919,7 +919,7 @@ __device__ bool ph_first_update(Ex &ex, const Graph &g, const Work &w, uint32_t 
             const NibUnit x = load_unit(w, in, u);
             const uint32_t both = x.live & x.fwd & x.bwd;
             if (both) mn = min(mn, u * 32u + (uint32_t)__ffs(both) - 1u);
-            count_verts_n(ex, in ? min(32u, g.V + 1u - u * 32u) : 0u);
+            count_verts_n(ex, __popc(x.live & ~both));   // the listed ones: the rest cost half a byte each
             unit_walk2(u, x.live & ~both, [&](const bool (&ok)[2], const uint32_t (&v)[2], const unsigned (&)[2]) {
                 bq_add_edges(0, (ok[0] ? __ldg(&g.Fr[v[0] + 1u]) - __ldg(&g.Fr[v[0]]) : 0u) +
                                     (ok[1] ? __ldg(&g.Fr[v[1] + 1u]) - __ldg(&g.Fr[v[1]]) : 0u));
