@@ -778,11 +778,19 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
     });
     if (!ok) return false;
     // The claims of a pass are tallied by degree (the frontier edges Beamer's
-    // rule weighs) only while they could reach the bottom-up threshold: a
-    // pass is taken to leave at most four times the edges of its frontier (and
-    // at most the scope), and each claim brings at most maxdeg edges.  Bit d of known: the previous
-    // pass tallied direction d, so its count is exact.  Whole-GPU policy
-    // only: the single-CTA and batched searches are short, and there the
+    // rule weighs) only while they could reach the bottom-up threshold: each
+    // claim brings at most maxdeg edges, and a pass of one level claims at most
+    // the edges of its frontier (and at most the scope).  A pass in which warps
+    // go on with their own finds can claim more; it is weighed by its frontier
+    // all the same, so a pass that should go bottom-up may come one pass later.
+    // That is rare (such a pass is not expected to grow, see spreads) and
+    // cheaper than the offset gathers: 2M random vertices of degree 8 behind a
+    // path of 500, vSlota, 1,161 us, tallied in every such pass 1,210; 4096^2
+    // grid 2,306 and 2,522.  Four times the frontier's edges, as a guess at what those
+    // passes claim, is no better either: 400,000 random vertices of degree 3
+    // 294 us, now 283; 4096^2 grid 2,438.
+    // Bit d of known: the previous pass tallied direction d, so its count is
+    // exact.  Whole-GPU policy only: the single-CTA and batched searches are short, and there the
     // extra registers cost more than the gathers they save.
     unsigned known = 3u;
     const uint32_t dmax32 = Ex::grid ? __ldcg(&ex.ctl->maxdeg) : 0u;
@@ -812,7 +820,7 @@ __device__ bool ph_bfs(Ex &ex, const Graph &g, const Work &w, uint32_t p, int lw
             for (int d = 0; d < 2; d++) {
                 const bool pu = d ? pub : puf;
                 const unsigned long long nfd = d ? nb : nf, mfd = d ? mb : mf, nhd = d ? nhb : nhf;
-                unsigned long long xe = pu ? nscope : 4u * ((((known >> d) & 1u) ? mfd : nfd * dmax) + nhd * CH);
+                unsigned long long xe = pu ? nscope : (((known >> d) & 1u) ? mfd : nfd * dmax) + nhd * CH;
                 xe = min(xe, (unsigned long long)nscope);
                 if (w.bu_k && xe * dmax > (unsigned long long)nscope * w.bu_k) cm |= 1u << d;
             }
