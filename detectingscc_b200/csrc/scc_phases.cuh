@@ -345,8 +345,8 @@ __device__ bool ph_init(Ex &ex, const Graph &g, const Work &w, bool trim, bool s
 
 // ---------------------------------------------------------------------
 // trim1 iterated to its fixpoint (vHong / wHong, scc_WCC.cu:680-687,
-// :773-780, :808-815).  Pass 0 checks a list or, without one, every live
-// vertex (by id, off the nibble units); a trimmed vertex queues its live neighbours of the
+// :773-780, :808-815).  Pass 0 checks every live vertex (all: by id, off the
+// nibble units, n of them) or a list; a trimmed vertex queues its live neighbours of the
 // same class for the next pass (stamped with the pass, so none is listed
 // twice; a vertex that is being checked meanwhile is listed all the same),
 // so later passes only recheck vertices that lost a neighbour.  A vertex is checked by searching both its lists for one live
@@ -407,15 +407,17 @@ __device__ __forceinline__ void trim1_check(Ex &ex, const Graph &g, const Work &
     }
 }
 
+// (all is a parameter of its own: with the choice made by the list's pointer
+// the three calls share code that spills, one CTA and 1,024 vertices 104 -> 115 us)
 template <class Ex>
-__device__ bool ph_trim1_fix(Ex &ex, const Graph &g, const Work &w, VList src0)
+__device__ bool ph_trim1_fix(Ex &ex, const Graph &g, const Work &w, VList src0, bool all)
 {
     uint32_t nq = src0.n;
     for (unsigned it = 0;; it++) {
         if (it > g.V + 2u) { if (ex.leader()) set_error(ex.ctl, E_NOT_CONVERGED, 30); return false; }
         const bool ok = run_pass(ex, PH_TRIM1_FIX, [&](unsigned, unsigned nxt) {
             const unsigned par = ex.gl & 1u;
-            if (!src0.p && it == 0u) {
+            if (all && it == 0u) {
                 const uint32_t nu = g.V / 32u + 1u, cu = unit_group(ex, g.V), ni = (nu + cu - 1u) / cu;
                 for (uint32_t i = ex.wid(); i < ni; i += ex.nwarps()) {
                     const uint32_t u = lane_id() * ni + i;
@@ -1523,7 +1525,7 @@ __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t
     uint32_t nlive = last_count(ex, C_LIST);
     unsigned long long k = vld64(&w.pivkey[0]);
     if (t1 && nlive) {
-        if (!ph_trim1_fix(ex, g, w, VList{nullptr, nlive})) return RUN_ERROR;
+        if (!ph_trim1_fix(ex, g, w, VList{nullptr, nlive}, true)) return RUN_ERROR;
         nlive = g.V - (uint32_t)vld64(&ex.ctl->n_trim1);
         if (nlive && !(nib_of(w.nb, key_vertex(k)) & NL)) {
             if (!ph_first_pivot(ex, g, w)) return RUN_ERROR;
@@ -1540,9 +1542,9 @@ __device__ int hong_front(Ex &ex, const Graph &g, const Work &w, bool t1, bool t
     cy.lsel = 1u;
     cy.nL = L1.n;
     cy.nE = last_count(ex, C_FE);
-    if (t1 && !ph_trim1_fix(ex, g, w, L1)) return RUN_ERROR;
+    if (t1 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
     if (t2 && !ph_trim2(ex, g, w, L1)) return RUN_ERROR;
-    if (t1 && t2 && !ph_trim1_fix(ex, g, w, L1)) return RUN_ERROR;
+    if (t1 && t2 && !ph_trim1_fix(ex, g, w, L1, false)) return RUN_ERROR;
     if (t1 || t2) {
         if (!ph_compact(ex, g, w, L1, w.L[0])) return RUN_ERROR;
         cy.lsel = 0u;
