@@ -302,7 +302,7 @@ def run_ours(args):
     B_alg = 8 * ins["edges_scanned"] + 12 * (ins["vertex_visits"] - V) + 9 * V
     peak, peak_kind = _peak_hbm()
     achieved = B_alg / (t_kern * 1e-3) / 1e9
-    tr = _traffic(args.config if args.scale is None else None)
+    tr = _traffic(args.config if args.scale is None and not args.permute else None)
     out = {
         "metric": f"SCC Medges/s ({'vSlota' if cfg['algo'] == 'h' else cfg['algo']}, {args.config})",
         "value": round(world * E / (t_step * 1e-3) / 1e6, 2),
