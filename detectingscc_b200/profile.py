@@ -12,9 +12,9 @@ the 126 MB L2, and each run holds a few GB of device memory at most.
         (k_parse_count, k_parse_write and the sorts above)
     python -m detectingscc_b200.profile scc --config cfg1|cfg2|cfg3 [--reps 2]
         one decomposition per rep (k_scc_block or k_scc_grid, k_canon_write)
-    python -m detectingscc_b200.profile batch [--graphs 256] [--reps 2]
+    python -m detectingscc_b200.profile batch [--graphs 256] [--cluster 4] [--reps 2]
         the batched form on the largest graphs of the 4,096-graph mix
-        (k_scc_batch), default schedule
+        (k_scc_batch), default schedule or the larger graphs on clusters
 
 Every run checks its result against the host-built CSR or the oracle-free
 invariants it can (derive: bit-exact reverse CSR; ingest: bit-exact CSRs;
@@ -121,6 +121,8 @@ def run_batch(args):
     gs = [scc.graph_from_arcs(*graphs.batch_mix_graph(i, seed=1)) for i in idx]
     eng = scc.Engine(0)
     b = scc.Batch(eng, gs)
+    if args.cluster:
+        b.set_cluster(args.cluster, 32768)
     try:
         n0 = None
         for r in range(args.reps):
@@ -141,6 +143,7 @@ def main():
     ap.add_argument("--scale", type=int, default=None)
     ap.add_argument("--config", default="cfg2", choices=["cfg1", "cfg2", "cfg3"])
     ap.add_argument("--graphs", type=int, default=256)
+    ap.add_argument("--cluster", type=int, default=0, help="CTAs of a cluster for graphs from 32,768 vertices on")
     ap.add_argument("--reps", type=int, default=2)
     args = ap.parse_args()
     {"derive": run_derive, "ingest": run_ingest, "scc": run_scc, "batch": run_batch}[args.what](args)
