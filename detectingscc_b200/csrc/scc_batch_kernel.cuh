@@ -79,7 +79,10 @@ __device__ void batch_one(Ex &ex, const BatchParams &p, uint32_t gi, char *base,
 // next[0] for cluster graphs, next[1] for CTA graphs.
 // CL: the variant with the cluster loop, launched only when the batch has
 // cluster graphs (kept apart so the common one-CTA-per-graph kernel does
-// not carry the cluster path's registers).
+// not carry the cluster path's registers).  64 registers a thread, so that an
+// SM holds 1,024 of them: spilled, bytes stored / loaded (-Xptxas -v): Slota
+// 16 / 20 and with clusters 160 / 808, Hong, whose trims share the frame with
+// the search and the peels, 184 / 160 and 540 / 1,712.
 template <int THREADS, bool HONG, bool CL>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_scc_batch(BatchParams p)
 {

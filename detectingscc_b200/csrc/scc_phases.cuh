@@ -982,8 +982,8 @@ __device__ bool ph_compact(Ex &ex, const Graph &g, const Work &w, VList src, uin
 // sweeps and levels together, and a third of the colour loop's arcs.  What
 // bounds them is the chain of dependent accesses of each level (list entry,
 // offsets and colour, arcs, neighbour's pair, atomic).  That graph, before
-// and now: one CTA vHong 26.5 -> 8.1 ms, vSlota 50.1 -> 6.8 ms; whole GPU
-// 18.6 -> 1.36 ms and 11.7 -> 1.26 ms.
+// and now: one CTA vHong 26.5 -> 7.3 ms, vSlota 50.1 -> 6.4 ms; whole GPU
+// 18.6 -> 1.22 ms and 11.7 -> 1.16 ms.
 //
 // A live vertex's word pair pc[v]: x the range, y = (colour << 1) | flag.
 // One 8-byte gather per arc decides; a word of a vertex without colour is

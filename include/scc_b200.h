@@ -164,7 +164,7 @@ int scc_derive_reverse(scc_context *ctx, const uint32_t *Fr, const uint32_t *Fc,
  *                         default 0: the hardware cluster barrier)
  *   "max_passes"          a run stops with SCC_ERR_NOT_CONVERGED once it has
  *                         made this many device passes (0, the default: no
- *                         cap beyond the V + 2 passes of every loop)
+ *                         cap beyond the 2 V + 4 passes of a search)
  *   "test_withhold_arrival"  failure-detection test hook: with k + 1, one CTA
  *                         of a whole-GPU launch (or of a cluster in check
  *                         mode) withholds its barrier arrival at pass k, so
